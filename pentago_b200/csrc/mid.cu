@@ -29,22 +29,39 @@
 
 namespace pg {
 
-// Threads of a CTA that solves one board alone (its tiles stay kMidThreads
-// set0 rows: the extra warps share the rows' items).
+// Threads of a CTA that solves one board alone.
 constexpr int kMidBoardThreads = 512;
 
+// Shared memory of a pass CTA: the rows of a whole level (at most 252 of 144
+// bytes with up to 10 empty spots), the workspace, and the per-level tables.
+constexpr int kSmallTile = 36 << 10;
+constexpr int kSmallTables = 46 << 10;   // 1,275 x 32 + 232 x 8 + 1,808 x 2 bytes for 10 empty spots
+constexpr size_t kPassSmem = kSmallTile + size_t(kSmemWorkspaceMax) * 16 + kSmallTables;
+
+// The descriptor is read throughout; shared memory keeps those reads short.
+__device__ __forceinline__ void load_job(mid_job_t& J, const mid_job_t& from) {
+  for (int i = threadIdx.x; i < int(sizeof(mid_job_t) / 16); i += blockDim.x)
+    reinterpret_cast<uint4*>(&J)[i] = reinterpret_cast<const uint4*>(&from)[i];
+}
+
+// One board per CTA, both passes; the workspace in shared memory or global.
+template<bool SMEM>
 __global__ void __launch_bounds__(kMidBoardThreads)
-mid_board_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict__ wf, int smem_workspace) {
-  const mid_job_t& J = jobs[blockIdx.x];
+mid_board_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict__ wf) {
   extern __shared__ uint4 smem[];
-  set0_info* tiles = reinterpret_cast<set0_info*>(smem);  // kMidThreads entries
-  uint4* ws = smem_workspace ? smem + kMidThreads * sizeof(set0_info) / sizeof(uint4) : J.workspace;
+  __shared__ mid_job_t J;
+  __shared__ mid_choose_smem choose;
   __shared__ uint4 raw[2][19];
   __shared__ int fault;
+  load_job(J, jobs[blockIdx.x]);
+  load_choose(choose);
   if (threadIdx.x == 0) fault = 0;
   __syncthreads();
-  const mid_tables MT = {c_choose, c_winpat, wf};
-  mid_board_body(J, MT, tiles, ws, raw, &fault, threadIdx.x, blockDim.x, 0, 1, sync_threads(), sync_threads());
+  constexpr int tile_bytes = SMEM ? kSmallTile : kTileBytes;
+  uint4* ws = SMEM ? smem + tile_bytes / sizeof(uint4) : J.workspace;
+  const mid_tables MT = {choose.row, c_winpat, wf};
+  mid_board_body(J, MT, reinterpret_cast<char*>(smem), ws, raw, &fault, threadIdx.x, blockDim.x, 0, 1, sync_threads(),
+                 sync_threads(), nullptr, 0, 2, true, tile_bytes);
 }
 
 // Where the two pass CTAs of one board meet: each publishes the n <= 1
@@ -59,24 +76,32 @@ struct pass_meet {
 
 // The boards of pg_midsolve_batch whose workspace fits shared memory: two
 // CTAs per board, CTA 2b + p running pass p (aggressive = p) of board b over
-// its own copy of the per-level tables (jobs[2b + p]).  The passes share no
+// its own per-level tables (in shared memory; jobs[2b + p]).  The passes share no
 // workspace, so neither CTA waits for the other: the one that finishes second
 // (an atomic count, no spinning) gathers both passes' results and runs the
 // traversal.  A 64-board batch thus spreads over 128 SMs instead of 64.
 __global__ void __launch_bounds__(kMidBoardThreads)
 mid_pass_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict__ wf, pass_meet* meet) {
   const int board = blockIdx.x >> 1, pass = blockIdx.x & 1;
-  const mid_job_t& J = jobs[blockIdx.x];
   extern __shared__ uint4 smem[];
-  set0_info* tiles = reinterpret_cast<set0_info*>(smem);  // kMidThreads entries
-  uint4* ws = smem + kMidThreads * sizeof(set0_info) / sizeof(uint4);
+  uint4* ws = smem + kSmallTile / sizeof(uint4);
+  __shared__ mid_job_t J;
+  __shared__ mid_choose_smem choose;
   __shared__ uint4 raw[2][19];
   __shared__ int fault, last;
+  load_job(J, jobs[blockIdx.x]);
+  load_choose(choose);
   if (threadIdx.x == 0) fault = 0;
   __syncthreads();
-  const mid_tables MT = {c_choose, c_winpat, wf};
-  mid_board_body(J, MT, tiles, ws, raw, &fault, threadIdx.x, blockDim.x, 0, 1, sync_threads(), sync_threads(),
-                 nullptr, pass, pass + 1, false);
+  if (threadIdx.x == 0) {
+    J.wins1 = ws + kSmemWorkspaceMax;
+    J.sets1p = reinterpret_cast<uint64_t*>(J.wins1 + 2 * J.wins1_off[J.spots + 1]);
+    J.cs1ps = reinterpret_cast<uint16_t*>(J.sets1p + J.sets1p_off[J.spots + 1]);
+  }
+  __syncthreads();
+  const mid_tables MT = {choose.row, c_winpat, wf};
+  mid_board_body(J, MT, reinterpret_cast<char*>(smem), ws, raw, &fault, threadIdx.x, blockDim.x, 0, 1, sync_threads(),
+                 sync_threads(), nullptr, pass, pass + 1, false, kSmallTile);
   pass_meet& M = meet[board];
   if (threadIdx.x < 19) M.raw[pass][threadIdx.x] = raw[pass][threadIdx.x];
   if (threadIdx.x == 0 && fault) atomicExch(&M.fault, 1);
@@ -90,12 +115,11 @@ mid_pass_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict__
     if (threadIdx.x == 0) { J.out->size = -1; J.out->pad = 0; }
     return;
   }
-  // Interleave (midengine.cc:119-124) and traverse on the first warp
-  uint4 supers[2 * 19];
-  for (int i = 0; i < 19; i++)
-    for (int j = 0; j < 2; j++) supers[2 * i + j] = __ldcg(&M.raw[j ^ (i == 0)][i]);
+  // The other pass's results beside this CTA's own, and traverse on the first warp
+  if (threadIdx.x < 19) raw[pass ^ 1][threadIdx.x] = __ldcg(&M.raw[pass ^ 1][threadIdx.x]);
+  __syncwarp();
 #ifdef __CUDA_ARCH__
-  traverse_warp(J, MT, supers, J.out, int(threadIdx.x));
+  traverse_warp(J, MT, raw, J.out, int(threadIdx.x));
 #endif
 }
 
@@ -112,24 +136,27 @@ __global__ void barrier_timeout_kernel(unsigned* words, int* fault, unsigned pol
 // A few large boards: ncta CTAs per board (blockIdx.x / ncta), each taking a
 // contiguous share of every level.  bar: 2 words per board; raw: 38 uint4 per
 // board; faults: one per board; all zero at launch.
-__global__ void __launch_bounds__(kMidThreads, 3)
+__global__ void __launch_bounds__(kMidThreads, 4)
 mid_board_grid_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict__ wf, int ncta, unsigned* bar,
                       uint4* rawg, int* faults) {
   const int board = blockIdx.x / ncta, cta = blockIdx.x % ncta;
-  const mid_job_t& J = jobs[board];
   extern __shared__ uint4 smem[];
-  set0_info* tiles = reinterpret_cast<set0_info*>(smem);
-  const mid_tables MT = {c_choose, c_winpat, wf};
+  __shared__ mid_job_t J;
+  __shared__ mid_choose_smem choose;
+  load_job(J, jobs[board]);
+  load_choose(choose);
+  __syncthreads();
+  const mid_tables MT = {choose.row, c_winpat, wf};
   const board_barrier gb{bar + 2 * board, bar + 2 * board + 1, ncta, faults + board};
-  mid_board_body(J, MT, tiles, J.workspace, reinterpret_cast<uint4(*)[19]>(rawg + 38 * board), faults + board,
-                 int(threadIdx.x), int(blockDim.x), cta, ncta, sync_threads(), gb);
+  mid_board_body(J, MT, reinterpret_cast<char*>(smem), J.workspace, reinterpret_cast<uint4(*)[19]>(rawg + 38 * board),
+                 faults + board, int(threadIdx.x), int(blockDim.x), cta, ncta, sync_threads(), gb);
 }
 
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 
-static uint32_t h_choose[19][11];
+static mid_choose h_choose[19];
 
 int hchoose(int n, int k) {
   if (n < 0 || k < 0 || k > n) return 0;
@@ -203,13 +230,15 @@ bool plan_board(uint64_t raw, board_plan& P, std::string& err) {
 }
 
 static int mid_kernel_attrs() {
-  const int smem_ws = int(kMidThreads * sizeof(set0_info) + kSmemWorkspaceMax * 16);
-  return cudaFuncSetAttribute(mid_board_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_ws) ==
+  const int smem_ws = int(kSmallTile + kSmemWorkspaceMax * 16);
+  return cudaFuncSetAttribute(mid_board_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_ws) ==
                      cudaSuccess &&
-                 cudaFuncSetAttribute(mid_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_ws) ==
+                 cudaFuncSetAttribute(mid_board_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kTileBytes) == cudaSuccess &&
+                 cudaFuncSetAttribute(mid_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPassSmem)) ==
                      cudaSuccess &&
                  cudaFuncSetAttribute(mid_board_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(kMidThreads * sizeof(set0_info))) == cudaSuccess
+                                      kTileBytes) == cudaSuccess
              ? 0 : PG_ERR_CUDA;
 }
 
@@ -361,17 +390,16 @@ extern "C" int pg_midsolve_batch(const uint64_t* raws, int n, pg_mid_values_t* o
   PG_CUDA(cudaMemcpyAsync(djobs, host_jobs.data(), jbytes, cudaMemcpyHostToDevice, stream));
   if (nsmall) {
     PG_CUDA(cudaMemsetAsync(meets, 0, sizeof(pass_meet) * size_t(nsmall), stream));
-    const size_t smem = kMidThreads * sizeof(set0_info) + kSmemWorkspaceMax * 16;
-    mid_pass_kernel<<<unsigned(2 * nsmall), kMidBoardThreads, smem, stream>>>(
+    mid_pass_kernel<<<unsigned(2 * nsmall), kMidBoardThreads, kPassSmem, stream>>>(
         reinterpret_cast<const mid_job_t*>(djobs), T->win_factors, meets);
     PG_CUDA(cudaGetLastError());
   }
   if (nlarge) {
     const mid_job_t* d = reinterpret_cast<const mid_job_t*>(djobs + small_jobs_bytes(nsmall));
-    const size_t smem = kMidThreads * sizeof(set0_info);
+    const size_t smem = size_t(kTileBytes);
     const int ncta = grid_ctas_per_board(nlarge, smem);
     if (ncta <= 1) {
-      mid_board_kernel<<<unsigned(nlarge), kMidBoardThreads, smem, stream>>>(d, T->win_factors, 0);
+      mid_board_kernel<false><<<unsigned(nlarge), kMidBoardThreads, smem, stream>>>(d, T->win_factors);
       PG_CUDA(cudaGetLastError());
     } else {
       if (int rc = launch_grid_boards(d, nlarge, ncta, smem, T->win_factors, grid_aux, stream)) return rc;
@@ -401,11 +429,11 @@ extern "C" int pg_debug_barrier_timeout(unsigned polls, int* fault_out) {
 // the midsolve arithmetic and indexing).  out: host array of n records.
 extern "C" int pg_selftest_midsolve_host(const uint64_t* raws, int n, pg_mid_values_t* out, uint64_t* supers) {
   for (int k = 0; k <= 18; k++)
-    for (int j = 0; j <= 10; j++) h_choose[k][j] = uint32_t(hchoose(k, j));
+    for (int j = 0; j < 20; j++) h_choose[k][j] = uint16_t(hchoose(k, j));
   const tables_t& T = tables();
   const mid_tables MT = {h_choose, T.winpat, &T.win_factors[0][0][0]};
   std::string err;
-  std::vector<set0_info> tiles(kMidThreads);
+  std::vector<uint4> tile(kTileBytes / sizeof(uint4));
   uint4 raw[2][19];
   for (int i = 0; i < n; i++) {
     board_plan P;
@@ -422,7 +450,7 @@ extern "C" int pg_selftest_midsolve_host(const uint64_t* raws, int n, pg_mid_val
     memset(raw, 0, sizeof raw);
     int fault = 0;
     J.ws_size = int(P.workspace);
-    mid_board_body(J, MT, tiles.data(), ws.data(), raw, &fault, 0, 1, 0, 1, [] {}, [] {},
+    mid_board_body(J, MT, reinterpret_cast<char*>(tile.data()), ws.data(), raw, &fault, 0, 1, 0, 1, [] {}, [] {},
                    supers ? reinterpret_cast<uint4*>(supers + 76 * size_t(i)) : nullptr);
   }
   return PG_OK;
@@ -452,7 +480,7 @@ struct host_barrier {
 extern "C" int pg_selftest_midsolve_groups_host(const uint64_t* raws, int n, int groups, pg_mid_values_t* out) {
   if (n < 0 || groups < 1 || groups > 64) return fail(PG_ERR_ARG, "bad arguments");
   for (int k = 0; k <= 18; k++)
-    for (int j = 0; j <= 10; j++) h_choose[k][j] = uint32_t(hchoose(k, j));
+    for (int j = 0; j < 20; j++) h_choose[k][j] = uint16_t(hchoose(k, j));
   const tables_t& T = tables();
   const mid_tables MT = {h_choose, T.winpat, &T.win_factors[0][0][0]};
   std::string err;
@@ -473,11 +501,11 @@ extern "C" int pg_selftest_midsolve_groups_host(const uint64_t* raws, int n, int
     memset(raw, 0, sizeof raw);
     int fault = 0;
     host_barrier hb(groups);
-    std::vector<std::vector<set0_info>> tiles(groups, std::vector<set0_info>(kMidThreads));
+    std::vector<std::vector<uint4>> tiles(groups, std::vector<uint4>(kTileBytes / sizeof(uint4)));
     std::vector<std::thread> threads;
     for (int g = 0; g < groups; g++)
       threads.emplace_back([&, g] {
-        mid_board_body(J, MT, tiles[g].data(), ws.data(), raw, &fault, 0, 1, g, groups, [] {}, [&] { hb.wait(); });
+        mid_board_body(J, MT, reinterpret_cast<char*>(tiles[g].data()), ws.data(), raw, &fault, 0, 1, g, groups, [] {}, [&] { hb.wait(); });
       });
     for (auto& t : threads) t.join();
   }
@@ -588,8 +616,9 @@ extern "C" int pg_midsolve_batch_noalloc(const uint64_t* raws, int n, pg_mid_val
     mid_job_t* d = reinterpret_cast<mid_job_t*>(pass ? large_dev : small_dev);
     PG_CUDA(cudaMemcpyAsync(d, jobs.data(), sizeof(mid_job_t) * jobs.size(), cudaMemcpyHostToDevice, stream));
     const int smem_ws = pass == 0;
-    const size_t smem = kMidThreads * sizeof(set0_info) + (smem_ws ? kSmemWorkspaceMax * 16 : 0);
-    mid_board_kernel<<<unsigned(jobs.size()), kMidBoardThreads, smem, stream>>>(d, D.win_factors, smem_ws);
+    const size_t smem = smem_ws ? kSmallTile + size_t(kSmemWorkspaceMax) * 16 : size_t(kTileBytes);
+    if (smem_ws) mid_board_kernel<true><<<unsigned(jobs.size()), kMidBoardThreads, smem, stream>>>(d, D.win_factors);
+    else mid_board_kernel<false><<<unsigned(jobs.size()), kMidBoardThreads, smem, stream>>>(d, D.win_factors);
     PG_CUDA(cudaGetLastError());
   }
   return PG_OK;

@@ -105,13 +105,15 @@ __global__ void __launch_bounds__(kMidThreads, 3)
 serve_kernel(serve_entry* ring, serve_ctl* ctl, serve_dev* dev, gang_aux* aux,
              const uint32_t* __restrict__ wf) {
   extern __shared__ uint4 smem[];
-  set0_info* tiles = reinterpret_cast<set0_info*>(smem);
+  char* tile = reinterpret_cast<char*>(smem);
   __shared__ uint4 raw[2][19];
   __shared__ int fault;
   __shared__ long long claimed;
   __shared__ mid_job_t job;
   __shared__ int gang_s, rank_s, first_s;
-  const mid_tables MT = {c_choose, c_winpat, wf};
+  __shared__ mid_choose_smem choose;
+  load_choose(choose);   // (every loop turn starts with a barrier)
+  const mid_tables MT = {choose.row, c_winpat, wf};
   for (;;) {
     if (threadIdx.x == 0) {
       claimed = -1;
@@ -157,7 +159,7 @@ serve_kernel(serve_entry* ring, serve_ctl* ctl, serve_dev* dev, gang_aux* aux,
     const mid_job_t& J = job;
     const int gang = gang_s, rank = rank_s, first = first_s;
     if (gang <= 1) {
-      mid_board_body(J, MT, tiles, J.workspace, raw, &fault, int(threadIdx.x), int(blockDim.x), 0, 1,
+      mid_board_body(J, MT, tile, J.workspace, raw, &fault, int(threadIdx.x), int(blockDim.x), 0, 1,
                      sync_threads(), sync_threads());
       __syncthreads();
       if (threadIdx.x == 0) {
@@ -169,7 +171,7 @@ serve_kernel(serve_entry* ring, serve_ctl* ctl, serve_dev* dev, gang_aux* aux,
       // gang are consecutive, so earlier requests never wait on later ones.
       gang_aux& X = aux[first];
       const board_barrier gb{&X.count, &X.gen, gang, &X.fault};
-      mid_board_body(J, MT, tiles, J.workspace, X.raw, &X.fault, int(threadIdx.x), int(blockDim.x), rank, gang,
+      mid_board_body(J, MT, tile, J.workspace, X.raw, &X.fault, int(threadIdx.x), int(blockDim.x), rank, gang,
                      sync_threads(), gb);
       __syncthreads();
       if (rank == 0 && threadIdx.x == 0) {
@@ -235,7 +237,7 @@ static int launch_workers(server& S) {
   if (!T) return PG_ERR_CUDA;
   S.ctl->close = 0;
   S.ctl->status = kRunning;
-  const size_t smem = kMidThreads * sizeof(set0_info);
+  const size_t smem = size_t(kTileBytes);
   PG_CUDA(cudaMemsetAsync(&S.dev->close, 0, sizeof(int), S.stream));
   serve_kernel<<<S.workers, kMidThreads, smem, S.stream>>>(S.ring, S.ctl, S.dev, S.aux, T->win_factors);
   PG_CUDA(cudaGetLastError());
@@ -257,9 +259,9 @@ extern "C" int pg_serve_open(int64_t budget_bytes, pg_server_t* out) {
   int sms = 0, per_sm = 0;
   PG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, S->device));
   PG_CUDA(cudaFuncSetAttribute(serve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(kMidThreads * sizeof(set0_info))));
+                               kTileBytes));
   PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, serve_kernel, kMidThreads,
-                                                        kMidThreads * sizeof(set0_info)));
+                                                        size_t(kTileBytes)));
   S->workers = sms * std::max(1, per_sm);
   PG_CUDA(cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking));
   PG_CUDA(cudaHostAlloc((void**)&S->ring, sizeof(serve_entry) * kRing, cudaHostAllocMapped));
