@@ -15,11 +15,13 @@
 // internal.h:174-259) is built cooperatively in shared memory.  Boards with
 // up to 10 empty spots (26 or more stones) keep their whole workspace in
 // shared memory (bottleneck(10) = 8400 halfsupers = 134 KB): in a batch, one
-// CTA per pass (mid_pass_kernel); larger boards use a global-memory
+// CTA per pass over index tables (mid_pass_kernel); larger boards use a global-memory
 // workspace.  The last step, midsolve_traverse (midengine.cc:127-158), also
 // runs on the device and writes the reference's mid_values_t records.
 #include "mid_body.cuh"
+#include "mid_small.cuh"
 #include "runtime.h"
+#include <cooperative_groups.h>
 #include <atomic>
 #include <algorithm>
 #include <condition_variable>
@@ -32,11 +34,14 @@ namespace pg {
 // Threads of a CTA that solves one board alone.
 constexpr int kMidBoardThreads = 512;
 
-// Shared memory of a pass CTA: the rows of a whole level (at most 252 of 144
-// bytes with up to 10 empty spots), the workspace, and the per-level tables.
+// Rows' room of a CTA that solves a board with up to 10 empty spots alone: a
+// whole level (at most 252 rows of 144 bytes).
 constexpr int kSmallTile = 36 << 10;
-constexpr int kSmallTables = 46 << 10;   // 1,275 x 32 + 232 x 8 + 1,808 x 2 bytes for 10 empty spots
-constexpr size_t kPassSmem = kSmallTile + size_t(kSmemWorkspaceMax) * 16 + kSmallTables;
+
+// Threads of a pass CTA, and its shared memory: the workspace and the wins.
+constexpr int kPassThreads = 768;
+constexpr int kPassWins = 2 * 1275 + 1;   // 10 empty spots
+constexpr size_t kPassSmem = (size_t(kSmemWorkspaceMax) + kPassWins) * 16;
 
 // The descriptor is read throughout; shared memory keeps those reads short.
 __device__ __forceinline__ void load_job(mid_job_t& J, const mid_job_t& from) {
@@ -64,62 +69,44 @@ mid_board_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict_
                  sync_threads(), nullptr, 0, 2, true, tile_bytes);
 }
 
-// Where the two pass CTAs of one board meet: each publishes the n <= 1
-// results of its pass (raw[pass][0..spots]) and its bounds-check fault, then
-// counts itself done; zero at launch.
-struct pass_meet {
-  uint4 raw[2][19];
-  unsigned done;
-  int fault;
-  int pad[2];
-};
-
-// The boards of pg_midsolve_batch whose workspace fits shared memory: two
-// CTAs per board, CTA 2b + p running pass p (aggressive = p) of board b over
-// its own per-level tables (in shared memory; jobs[2b + p]).  The passes share no
-// workspace, so neither CTA waits for the other: the one that finishes second
-// (an atomic count, no spinning) gathers both passes' results and runs the
-// traversal.  A 64-board batch thus spreads over 128 SMs instead of 64.
-__global__ void __launch_bounds__(kMidBoardThreads)
-mid_pass_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict__ wf, pass_meet* meet) {
-  const int board = blockIdx.x >> 1, pass = blockIdx.x & 1;
+// The boards of pg_midsolve_batch whose workspace fits shared memory: a
+// cluster of two CTAs per board, CTA p running pass p (aggressive = p) over the
+// index tables of its count of empty spots, so that 64 boards use 128 SMs.
+// Each CTA computes half of the wins for both; the passes share nothing else
+// until CTA 0 has the results of both and writes the records.  Bound by
+// the items: integer instructions (rmax, at half rate), conflicts of the
+// gathers from shared memory, and 11 barriers, about evenly.  64 boards of
+// 26 stones: 97 us with the indexes worked out by each CTA, 38 us now (passes
+// 28, wins 5; 512 and 1,024 threads within 2 us of this).
+__global__ void __cluster_dims__(2) __launch_bounds__(kPassThreads)
+mid_pass_kernel(const small_job* __restrict__ jobs, const uint32_t* __restrict__ wf,
+                const small_table* __restrict__ tables) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int pass = int(cluster.block_rank()), tid = threadIdx.x;
   extern __shared__ uint4 smem[];
-  uint4* ws = smem + kSmallTile / sizeof(uint4);
-  __shared__ mid_job_t J;
-  __shared__ mid_choose_smem choose;
+  uint4* ws = smem;
+  uint4* wins = smem + kSmemWorkspaceMax;
+  __shared__ small_job J;
+  __shared__ small_table T;
   __shared__ uint4 raw[2][19];
-  __shared__ int fault, last;
-  load_job(J, jobs[blockIdx.x]);
-  load_choose(choose);
-  if (threadIdx.x == 0) fault = 0;
+  const small_job& from = jobs[blockIdx.x >> 1];
+  if (tid < int(sizeof J / 8)) reinterpret_cast<uint64_t*>(&J)[tid] = reinterpret_cast<const uint64_t*>(&from)[tid];
+  const small_table* table = tables + from.spots;
+  for (int i = tid; i < int(sizeof T / 8); i += blockDim.x)
+    reinterpret_cast<uint64_t*>(&T)[i] = reinterpret_cast<const uint64_t*>(table)[i];
+  cluster.sync();   // (the other CTA has begun)
+  uint4* others = cluster.map_shared_rank(wins, pass ^ 1);
+  small_wins(J, wf, T, pass * blockDim.x + tid, 2 * blockDim.x, [&](int i, const uint4& v) { wins[i] = others[i] = v; });
+  cluster.sync();
+  small_pass(T, pass, ws, wins, raw[pass], tid, blockDim.x, sync_threads());
   __syncthreads();
-  if (threadIdx.x == 0) {
-    J.wins1 = ws + kSmemWorkspaceMax;
-    J.sets1p = reinterpret_cast<uint64_t*>(J.wins1 + 2 * J.wins1_off[J.spots + 1]);
-    J.cs1ps = reinterpret_cast<uint16_t*>(J.sets1p + J.sets1p_off[J.spots + 1]);
-  }
-  __syncthreads();
-  const mid_tables MT = {choose.row, c_winpat, wf};
-  mid_board_body(J, MT, reinterpret_cast<char*>(smem), ws, raw, &fault, threadIdx.x, blockDim.x, 0, 1, sync_threads(),
-                 sync_threads(), nullptr, pass, pass + 1, false, kSmallTile);
-  pass_meet& M = meet[board];
-  if (threadIdx.x < 19) M.raw[pass][threadIdx.x] = raw[pass][threadIdx.x];
-  if (threadIdx.x == 0 && fault) atomicExch(&M.fault, 1);
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&M.done, 1u) == 1u;
-  __syncthreads();
-  if (!last || threadIdx.x >= 32) return;
-  __threadfence();
-  if (atomicAdd(&M.fault, 0)) {
-    if (threadIdx.x == 0) { J.out->size = -1; J.out->pad = 0; }
-    return;
-  }
-  // The other pass's results beside this CTA's own, and traverse on the first warp
-  if (threadIdx.x < 19) raw[pass ^ 1][threadIdx.x] = __ldcg(&M.raw[pass ^ 1][threadIdx.x]);
-  __syncwarp();
+  if (pass && tid <= T.spots) *cluster.map_shared_rank(&raw[1][tid], 0) = raw[1][tid];
+  cluster.sync();
+  const int warp = tid >> 5;
+  if (pass || warp >= 3) return;   // (12 children at once)
 #ifdef __CUDA_ARCH__
-  traverse_warp(J, MT, raw, J.out, int(threadIdx.x));
+  traverse_warps(J.side, J.ply, c_winpat, raw, J.out, warp, 3, tid & 31);
 #endif
 }
 
@@ -242,6 +229,126 @@ static int mid_kernel_attrs() {
              ? 0 : PG_ERR_CUDA;
 }
 
+static small_job small_job_of(const mid_job_t& J) {
+  small_job S = {};
+  S.side[0] = J.side[0];
+  S.side[1] = J.side[1];
+  S.ply = J.ply;
+  S.spots = J.spots;
+  memcpy(S.empty, J.empty, sizeof S.empty);
+  S.out = J.out;
+  return S;
+}
+
+// Index tables of boards with up to kSmallSpots empty spots (mid_small.cuh),
+// from the definitions: a level's entry is the rank of one side's subset among
+// the spots and of the other's among those the first leaves free.
+const small_tables_host& small_tables() {
+  static const small_tables_host* H = [] {
+    auto* h = new small_tables_host;
+    auto rank = [](uint32_t set) {   // in large-entry-major order
+      int r = 0, i = 0;
+      for (int v = 0; v < 32; v++)
+        if (set >> v & 1) r += hchoose(v, ++i);
+      return r;
+    };
+    auto among = [](uint32_t set, uint32_t others) {   // set's spots counted without the others'
+      uint32_t r = 0;
+      for (int v = 0, k = 0; v < 32; v++)
+        if (!(others >> v & 1)) r |= (set >> v & 1) << k++;
+      return r;
+    };
+    for (int spots = 0; spots <= kSmallSpots; spots++) {
+      small_table& T = h->table[spots];
+      memset(&T, 0, sizeof T);
+      T.spots = spots;
+      h->rec0[spots] = h->recs.size();
+      h->child0[spots] = h->children.size();
+      h->subset0[spots] = h->subsets.size();
+      const int ws = bottleneck(spots);
+      std::vector<std::vector<uint32_t>> subsets(spots + 1);   // by size, in rank order
+      for (int k = 0; k <= spots; k++) {
+        subsets[k].resize(hchoose(spots, k));
+        for (uint32_t m = 0; m < 1u << spots; m++)
+          if (__builtin_popcount(m) == k) subsets[k][rank(m)] = m;
+      }
+      auto ny = [&](int n) { return hchoose(spots - (n - (n >> 1)), n >> 1); };   // entries per s1 of level n
+      for (int n = 0; n <= spots; n++) {
+        const int k0 = n >> 1, k1 = n - k0;
+        T.lo[n] = n & 1 ? ws - int(subsets[k1].size()) * ny(n) : 0;
+        T.wins[n] = T.nwins;
+        T.nwins += int(subsets[k1].size());
+        for (uint32_t m : subsets[k1]) h->subsets.push_back(uint16_t(m | uint32_t(n) << 10));
+        // items: every side-0 subset with every side-1 subset of the rest, in the order of both ranks
+        std::vector<std::pair<uint32_t, uint32_t>> items;
+        for (uint32_t set0 : subsets[k0]) {
+          std::vector<uint32_t> free1(hchoose(spots - k0, k1));
+          for (uint32_t set1 : subsets[k1])
+            if (!(set0 & set1)) free1[rank(among(set1, set0))] = set1;
+          for (uint32_t set1 : free1) items.emplace_back(set0, set1);
+        }
+        T.items[n] = int(items.size());
+        T.rec[n] = int(h->recs.size() - h->rec0[spots]);
+        T.child[n] = int(h->children.size() - h->child0[spots]);
+        h->children.resize(h->children.size() + items.size() * size_t(spots - n));
+        for (size_t it = 0; it < items.size(); it++) {
+          const uint32_t set0 = items[it].first, set1 = items[it].second;
+          const int o = rank(set1) * ny(n) + rank(among(set0, set1));
+          h->recs.push_back(uint32_t(o) | uint32_t(rank(set0)) << 13 | uint32_t(rank(set1)) << 21);
+          int c = 0;
+          for (int v = 0; v < spots; v++) {
+            if ((set0 | set1) >> v & 1) continue;
+            // the mover's stone at v: set0 with it is level n + 1's side 1
+            const uint32_t with = set0 | 1u << v;
+            h->children[h->child0[spots] + T.child[n] + size_t(c++) * items.size() + it] =
+                uint16_t(rank(with) * ny(n + 1) + rank(among(set1, with)));
+          }
+        }
+      }
+    }
+    for (int spots = 0; spots <= kSmallSpots; spots++) {
+      small_table& T = h->table[spots];
+      T.recs = h->recs.data() + h->rec0[spots];
+      T.children = h->children.data() + h->child0[spots];
+      T.subsets = h->subsets.data() + h->subset0[spots];
+    }
+    return h;
+  }();
+  return *H;
+}
+
+// Their copies on each device.
+static small_table* small_dev[64];
+static int upload_small_tables() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return PG_ERR_CUDA;
+  const small_tables_host& H = small_tables();
+  uint32_t* recs = nullptr;
+  uint16_t *children = nullptr, *subsets = nullptr;
+  small_table* tables = nullptr;
+  const size_t rb = H.recs.size() * sizeof(uint32_t), cb = H.children.size() * sizeof(uint16_t),
+               sb = H.subsets.size() * sizeof(uint16_t);
+  small_table T[kSmallSpots + 1];
+  bool ok = cudaMalloc(&recs, rb) == cudaSuccess && cudaMalloc(&children, cb) == cudaSuccess &&
+            cudaMalloc(&subsets, sb) == cudaSuccess && cudaMalloc(&tables, sizeof T) == cudaSuccess;
+  for (int s = 0; s <= kSmallSpots && ok; s++) {
+    T[s] = H.table[s];
+    T[s].recs = recs + H.rec0[s];
+    T[s].children = children + H.child0[s];
+    T[s].subsets = subsets + H.subset0[s];
+  }
+  ok = ok && cudaMemcpy(recs, H.recs.data(), rb, cudaMemcpyHostToDevice) == cudaSuccess &&
+       cudaMemcpy(children, H.children.data(), cb, cudaMemcpyHostToDevice) == cudaSuccess &&
+       cudaMemcpy(subsets, H.subsets.data(), sb, cudaMemcpyHostToDevice) == cudaSuccess &&
+       cudaMemcpy(tables, T, sizeof T, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (!ok) {
+    for (void* p : {(void*)recs, (void*)children, (void*)subsets, (void*)tables}) if (p) cudaFree(p);
+    return PG_ERR_CUDA;
+  }
+  small_dev[dev] = tables;
+  return PG_OK;
+}
+
 static int upload_consts() {
   if (int rc = mid_prepare_device()) return rc;
   return per_device_once((const void*)&mid_kernel_attrs, mid_kernel_attrs);
@@ -295,23 +402,21 @@ void carve_scratch(board_plan& P, char* base, bool global_ws) {
   J.workspace = global_ws || P.workspace > size_t(kSmemWorkspaceMax) ? (uint4*)(base + off) : nullptr;
 }
 
-// pg_midsolve_batch's scratch: the pass_meet records of the shared-memory
-// boards, the job descriptors (two per shared-memory board, one per pass
-// CTA, then one per larger board), the grid kernel's per-board words, then
-// per board its tables (twice for a
-// shared-memory board: one copy per pass CTA) and, for a larger board, its
-// global workspace.  With the caller's scratch, nothing is allocated.
+// pg_midsolve_batch's scratch: job descriptors, the grid kernel's per-board
+// words, then per larger board its tables and global workspace.  With the
+// caller's scratch, nothing is allocated.  (A shared-memory board needs its
+// descriptor alone; its size here is what callers have been told so far, so
+// that their buffers stay the right ones.)
 static bool smem_board(const board_plan& P) { return P.workspace <= size_t(kSmemWorkspaceMax); }
 static size_t batch_bytes_of(const board_plan& P) { return (smem_board(P) ? 2 : 1) * scratch_bytes_of(P); }
-static size_t meet_bytes(int nsmall) { return align256(sizeof(pass_meet) * size_t(nsmall)); }
-static size_t small_jobs_bytes(int nsmall) { return align256(sizeof(mid_job_t) * 2 * size_t(nsmall)); }
+static size_t small_jobs_bytes(int nsmall) { return align256(sizeof(small_job) * size_t(nsmall)); }
 static size_t jobs_bytes(int nsmall, int nlarge) {
   return small_jobs_bytes(nsmall) + align256(sizeof(mid_job_t) * size_t(nlarge));
 }
-// Everything before the boards' tables: pass_meet records, job descriptors
-// and the grid kernel's per-board words.
+// Everything before the boards' tables.
 static size_t head_bytes(int nsmall, int nlarge) {
-  return meet_bytes(nsmall) + jobs_bytes(nsmall, nlarge) + (nlarge ? grid_aux_bytes(nlarge) : 0);
+  return align256(624 * size_t(nsmall)) + align256(sizeof(mid_job_t) * 2 * size_t(nsmall)) +
+         align256(sizeof(mid_job_t) * size_t(nlarge)) + (nlarge ? grid_aux_bytes(nlarge) : 0);
 }
 
 }  // namespace pg
@@ -358,7 +463,7 @@ extern "C" int pg_midsolve_batch(const uint64_t* raws, int n, pg_mid_values_t* o
     nsmall += smem_board(plans[i]);
   }
   const int nlarge = n - nsmall;
-  const size_t head = meet_bytes(nsmall), jbytes = jobs_bytes(nsmall, nlarge);
+  const size_t jbytes = jobs_bytes(nsmall, nlarge);
   total += head_bytes(nsmall, nlarge);
   stream_scratch X(stream);
   char* base = (char*)scratch;
@@ -367,35 +472,35 @@ extern "C" int pg_midsolve_batch(const uint64_t* raws, int n, pg_mid_values_t* o
   } else if (size_t(scratch_bytes) < total) {
     return fail(PG_ERR_CAPACITY, "midsolve scratch too small");
   }
-  pass_meet* meets = reinterpret_cast<pass_meet*>(base);
-  // The job descriptors in the layout they take on the device, copied in one
-  // piece: small boards' pass jobs (board b at 2b, 2b + 1), then large boards.
+  // The job descriptors in the layout they take on the device, copied in one piece.
   std::vector<char> host_jobs(jbytes);
-  mid_job_t* small = reinterpret_cast<mid_job_t*>(host_jobs.data());
+  small_job* small = reinterpret_cast<small_job*>(host_jobs.data());
   mid_job_t* large = reinterpret_cast<mid_job_t*>(host_jobs.data() + small_jobs_bytes(nsmall));
-  char* grid_aux = base + head + jbytes;
+  char* grid_aux = base + jbytes;
   size_t off = head_bytes(nsmall, nlarge);
   for (int i = 0, ns = 0, nl = 0; i < n; i++) {
     auto& P = plans[i];
     P.job.out = out + i;
-    const size_t bytes = scratch_bytes_of(P);
-    for (int copy = 0; copy < (smem_board(P) ? 2 : 1); copy++) {
+    if (smem_board(P)) {
+      small[ns++] = small_job_of(P.job);
+    } else {
       carve_scratch(P, base + off);
-      off += bytes;
-      if (smem_board(P)) small[ns++] = P.job;
-      else large[nl++] = P.job;
+      off += scratch_bytes_of(P);
+      large[nl++] = P.job;
     }
   }
-  char* djobs = base + head;
-  PG_CUDA(cudaMemcpyAsync(djobs, host_jobs.data(), jbytes, cudaMemcpyHostToDevice, stream));
+  PG_CUDA(cudaMemcpyAsync(base, host_jobs.data(), jbytes, cudaMemcpyHostToDevice, stream));
   if (nsmall) {
-    PG_CUDA(cudaMemsetAsync(meets, 0, sizeof(pass_meet) * size_t(nsmall), stream));
-    mid_pass_kernel<<<unsigned(2 * nsmall), kMidBoardThreads, kPassSmem, stream>>>(
-        reinterpret_cast<const mid_job_t*>(djobs), T->win_factors, meets);
+    int dev = 0;
+    PG_CUDA(cudaGetDevice(&dev));
+    if (int rc = per_device_once((const void*)&upload_small_tables, upload_small_tables))
+      return fail(rc, "midsolve index table upload failed");
+    mid_pass_kernel<<<unsigned(2 * nsmall), kPassThreads, kPassSmem, stream>>>(reinterpret_cast<const small_job*>(base),
+                                                                               T->win_factors, small_dev[dev]);
     PG_CUDA(cudaGetLastError());
   }
   if (nlarge) {
-    const mid_job_t* d = reinterpret_cast<const mid_job_t*>(djobs + small_jobs_bytes(nsmall));
+    const mid_job_t* d = reinterpret_cast<const mid_job_t*>(base + small_jobs_bytes(nsmall));
     const size_t smem = size_t(kTileBytes);
     const int ncta = grid_ctas_per_board(nlarge, smem);
     if (ncta <= 1) {
@@ -452,6 +557,18 @@ extern "C" int pg_selftest_midsolve_host(const uint64_t* raws, int n, pg_mid_val
     J.ws_size = int(P.workspace);
     mid_board_body(J, MT, reinterpret_cast<char*>(tile.data()), ws.data(), raw, &fault, 0, 1, 0, 1, [] {}, [] {},
                    supers ? reinterpret_cast<uint4*>(supers + 76 * size_t(i)) : nullptr);
+    if (J.spots <= kSmallSpots) {
+      // the pass kernel's own code, over the index tables, gives the same
+      const small_table& S = small_tables().table[J.spots];
+      const small_job SJ = small_job_of(J);
+      std::vector<uint4> wins(2 * S.nwins + 1), results(J.spots + 1);
+      small_wins(SJ, MT.wf, S, 0, 1, [&](int i, const uint4& v) { wins[i] = v; });
+      for (int pass = 0; pass < 2; pass++) {
+        small_pass(S, pass, ws.data(), wins.data(), results.data(), 0, 1, [] {});
+        if (memcmp(results.data(), raw[pass], sizeof(uint4) * results.size()))
+          return fail(PG_ERR_BOUNDS, "the index tables give another result");
+      }
+    }
   }
   return PG_OK;
 }

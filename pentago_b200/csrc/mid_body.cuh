@@ -364,83 +364,75 @@ PG_HD void traverse(const mid_job_t& J, const mid_tables& MT, const uint4* super
 }
 
 #ifdef __CUDA_ARCH__
-// traverse on one warp: the root's children (one per lane) at once, their
-// records placed by a prefix sum over the lanes in the order traverse
-// writes them.
-__device__ void put_record(pg_mid_values_t* out, int k, uint64_t raw, int v) {
+// traverse on the device, by one warp or several (each works the layout out
+// for itself, and they share the records): lane p holds the p-th five-in-a-row
+// mask, so whether a side has won is a vote, and the cells that would complete
+// a five are one reduction; lane s holds the root's s-th child, whose records
+// start 9 places on per child before it, 8 fewer for each that is done.
+__device__ __forceinline__ void put_record(pg_mid_values_t* out, int k, uint64_t raw, int v) {
   if (k < 163) { out->entries[k].raw = raw; out->entries[k].value = v; out->entries[k].pad = 0; }
 }
-// The 8 rotation children of sd (8 records at out[at..]); returns their best value for the mover.
-__device__ int middle_children_at(const uint64_t* sd, uint32_t p, const uint4& r0, const uint4& r1,
-                                  pg_mid_values_t* out, int at) {
-  int best = -1;
-  const uint64_t board = board_of(sd[0], sd[1]);
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    const int q = s >> 1, d = (s & 1) ? -1 : 1;
-    const int idx = ((d & 3) << (2 * q)) >> 1;
-    const int v = hbit(r0, idx) + hbit(r1, idx) - 1;
-    put_record(out, at + s, rotated_board(board, sd, q, d) | uint64_t((p + 1) & 1) << 63, v);
-    best = best > -v ? best : -v;
-  }
-  return best;
+// The value of rotation s (quadrant s >> 1, left or right) from its parent's results.
+__device__ __forceinline__ int rotation_value(const uint4& r0, const uint4& r1, int s) {
+  const int idx = (((s & 1) ? 3 : 1) << (s & 6)) >> 1;
+  return hbit(r0, idx) + hbit(r1, idx) - 1;
+}
+__device__ __forceinline__ uint64_t rotation_board(const uint64_t* side, int s) {
+  return rotated_board(board_of(side[0], side[1]), side, s >> 1, (s & 1) ? -1 : 1);
 }
 // raw: both passes' n <= 1 results, interleaved as (win, notlose) of entry i
 // = raw[i == 0], raw[i != 0] at i (midengine.cc:119-124).
-__device__ void traverse_warp(const mid_job_t& J, const mid_tables& MT, const uint4 (*raw)[19], pg_mid_values_t* out,
-                              int lane) {
+__device__ void traverse_warps(const uint64_t* root, uint32_t ply, const uint64_t* winpat, const uint4 (*raw)[19],
+                               pg_mid_values_t* out, int warp, int warps, int lane) {
   const unsigned full = 0xffffffffu;
-  const uint64_t side[2] = {J.side[0], J.side[1]};
-  const uint32_t ply = J.ply;
-  int value = 0, total = 0;
-  if (done_value(MT, side, ply, &value)) {
+  const uint64_t side[2] = {root[0], root[1]};
+  const int turn = int(ply >> 1 & 1);
+  const uint64_t pattern = winpat[lane];
+  const bool bw = __any_sync(full, (side[0] & pattern) == pattern), ww = __any_sync(full, (side[1] & pattern) == pattern);
+  int value, total = 0;
+  if (bw || ww || ply == 72) {   // done_value
+    value = bw == ww ? 0 : bw == !turn ? 1 : -1;
   } else if (!(ply & 1)) {
-    // lane s: the s-th empty cell (at most 18)
-    const uint64_t empty = 0x01ff01ff01ff01ffull ^ side[0] ^ side[1];
+    // The children: a stone of the side to move on each empty cell (at most 18)
+    const uint64_t empty = 0x01ff01ff01ff01ffull ^ side[0] ^ side[1], missing = pattern & ~side[turn];
+    const bool one = (missing & (missing - 1)) == 0;
+    const uint64_t fives = uint64_t(__reduce_or_sync(full, one ? uint32_t(missing >> 32) : 0u)) << 32 |
+                           __reduce_or_sync(full, one ? uint32_t(missing) : 0u);
     const int nempty = __popcll(empty);
-    int cnt = 0, cv = -1;
-    uint64_t cs[2] = {side[0], side[1]};
-    if (lane < nempty) {
-      uint64_t e = empty;
-      for (int i = 0; i < lane; i++) e &= e - 1;
-      cs[(ply >> 1) & 1] |= e & (~e + 1);
-      cnt = done_value(MT, cs, ply + 1, &cv) ? 1 : 9;
+    uint64_t e = empty;
+    for (int i = 0; i < lane; i++) e &= e - 1;
+    const uint64_t stone = e & (~e + 1);   // (0 beyond the last child)
+    const bool wins = (stone & fives) != 0;
+    const unsigned won = __ballot_sync(full, wins);
+    total = 9 * nempty - 8 * __popc(won);
+    int cv = -1;
+    if (wins) cv = 1;
+    else if (lane < nempty) {
+      const uint4 r0 = raw[0][lane + 1], r1 = raw[1][lane + 1];
+#pragma unroll
+      for (int s = 0; s < 8; s++) cv = max(cv, -rotation_value(r0, r1, s));
     }
-    int incl = cnt;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(full, incl, o);
-      if (lane >= o) incl += v;
+    value = __reduce_max_sync(full, cv);
+    for (int c0 = 4 * warp; c0 < nempty; c0 += 4 * warps) {   // four children's rotations at once
+      const int c = c0 + (lane >> 3), s = lane & 7;
+      const uint64_t cstone = __shfl_sync(full, stone, c & 31);
+      const int ccv = __shfl_sync(full, cv, c & 31);
+      if (c >= nempty) continue;
+      uint64_t cs[2] = {side[0], side[1]};
+      cs[turn] |= cstone;
+      const int at = 9 * c - 8 * __popc(won & ((1u << c) - 1));
+      const bool done = won >> c & 1;
+      if (!done) put_record(out, at + s, rotation_board(cs, s), rotation_value(raw[0][c + 1], raw[1][c + 1], s));
+      if (s == 0) put_record(out, at + (done ? 0 : 8), board_of(cs[0], cs[1]) | uint64_t(1) << 63, ccv);
     }
-    const int base = incl - cnt;
-    total = __shfl_sync(full, incl, 31);
-    if (lane < nempty) {
-      if (cnt == 9) cv = middle_children_at(cs, ply + 1, raw[0][lane + 1], raw[1][lane + 1], out, base);
-      put_record(out, base + cnt - 1, board_of(cs[0], cs[1]) | uint64_t(1) << 63, cv);
-    }
-    int v = cv;
-    for (int o = 16; o; o >>= 1) {
-      const int w = __shfl_xor_sync(full, v, o);
-      v = v > w ? v : w;
-    }
-    value = v;
   } else {
     // lanes 0..7: the root's 8 rotation children
-    int best = -1;
-    if (lane < 8) {
-      const int q = lane >> 1, d = (lane & 1) ? -1 : 1;
-      const int idx = ((d & 3) << (2 * q)) >> 1;
-      const int v = hbit(raw[1][0], idx) + hbit(raw[0][0], idx) - 1;
-      put_record(out, lane, rotated_board(board_of(side[0], side[1]), side, q, d) | uint64_t((ply + 1) & 1) << 63, v);
-      best = -v;
-    }
-    for (int o = 16; o; o >>= 1) {
-      const int w = __shfl_xor_sync(full, best, o);
-      best = best > w ? best : w;
-    }
-    value = best;
+    const int v = rotation_value(raw[1][0], raw[0][0], lane & 7);
+    if (warp == 0 && lane < 8) put_record(out, lane, rotation_board(side, lane), v);
+    value = __reduce_max_sync(full, -v);
     total = 8;
   }
-  if (lane == 0) {
+  if (warp == 0 && lane == 0) {
     put_record(out, total, board_of(side[0], side[1]) | uint64_t(ply & 1) << 63, value);
     out->size = total + 1;
     out->pad = 0;
@@ -562,7 +554,7 @@ PG_HD void mid_board_body(const mid_job_t& J, const mid_tables& MT, char* tile, 
   if (gtid == 0 && *fault) { J.out->size = -1; J.out->pad = 0; }
 #ifdef __CUDA_ARCH__
   // the first warp traverses (nt >= 32 on the device)
-  if (gtid < 32 && !*fault) traverse_warp(J, MT, raw, J.out, gtid);
+  if (gtid < 32 && !*fault) traverse_warps(J.side, J.ply, MT.winpat, raw, J.out, 0, 1, gtid);
 #else
   if (gtid == 0 && !*fault) {
     uint4 supers[2 * 19];

@@ -23,3 +23,13 @@ def test_mixed_batch_matches_oracle(cuda, O, stones):
     raws = np.concatenate([raws, raws[::-1] | np.uint64(1 << 63)])
     for raw, g in zip(raws, mid.midsolve(raws)):
         assert g == oracle_values(O, raw), f"board {int(raw)}"
+
+
+def test_more_small_boards_than_fit_at_once(cuda, O):
+    """Every size of board that is solved over index tables, in a batch of
+    more cluster pairs than the GPU holds at once."""
+    from pentago_b200 import mid
+    raws = np.concatenate([mid.random_boards(400 + s, 30 if s > 28 else 3, s) for s in range(26, 37)])
+    raws[1::2] |= np.uint64(1 << 63)
+    for raw, g in zip(raws, mid.midsolve(raws)):
+        assert g == oracle_values(O, raw), f"board {int(raw)}"
