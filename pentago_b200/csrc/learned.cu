@@ -2,7 +2,7 @@
 // kernels that train its network.  The model and the exact arithmetic of the
 // coding path are specified in learned.cuh.
 //
-// Coder layout: one warp per stream; lane l codes the run of nodes l R ..
+// Coder layout: 32 lanes per stream; lane l codes the run of nodes l R ..
 // l R + R - 1 (R = ceil(n / 32)), node l R + k in round k, its own rANS
 // state walking the steps (round, rotation) in order.  The encoder runs the
 // steps backward; at each step the lanes that renormalize append one 16-bit
@@ -35,11 +35,10 @@ constexpr int kLmWarps = 4;
 constexpr int kLmThreads = 32 * kLmWarps;
 constexpr int kLmCtxRows = kLmIn - kLmRot;   // W1 rows 72..123: the rotation, neighbour and previous-node features
 
-// Coding tables in shared memory.  The tensor cores' B operands are stored
-// transposed, one row of 64 bf16 (8 chunks of 16 bytes) per output unit:
-// w1t row k holds W1[72 + 8 c .. 72 + 8 c + 7][k] in chunk c (c < 6), w2t
-// row j holds W2[8 c .. 8 c + 7][j], chunk c at c ^ (row & 7) so that the
-// eight rows an ldmatrix phase reads fall in different banks.
+// Tables of the frequency check kernel in shared memory, transposed: one row
+// of 64 bf16 (8 chunks of 16 bytes) per output unit, w1t row k with
+// W1[72 + 8 c .. 72 + 8 c + 7][k] in chunk c (c < 7), w2t row j with
+// W2[8 c .. 8 c + 7][j], chunk c at c ^ (row & 7).
 struct lm_tables {
   uint4 w1t[kLmHidden][8];
   uint4 w2t[kLmHidden][8];
@@ -86,10 +85,10 @@ __device__ __forceinline__ float lm_tab(const uint4 (*tab)[8], int row, int k) {
 // node[k] = b1[k] + stone rows, ascending (registers of one thread); the
 // stone rows are read from the model (bf16, global memory: a lane reads them
 // once per node).
-__device__ __forceinline__ void lm_node_sum(const lm_tables& S, const uint16_t* __restrict__ P, const uint8_t* feats,
+__device__ __forceinline__ void lm_node_sum(const float* b1, const uint16_t* __restrict__ P, const uint8_t* feats,
                                             int nf, float* node) {
 #pragma unroll
-  for (int k = 0; k < kLmHidden; k++) node[k] = S.b1[k];
+  for (int k = 0; k < kLmHidden; k++) node[k] = b1[k];
   for (int i = 0; i < nf; i++) {
     const uint4* row = reinterpret_cast<const uint4*>(P + kLmW1 + feats[i] * kLmHidden);
 #pragma unroll
@@ -157,152 +156,242 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// out[n] += A x B for the eight n-tiles of a transposed table, k-tile kt.
-__device__ __forceinline__ void mma_row(float (*acc)[4], const uint32_t* a, const uint4 (*tab)[8], int kt, int lane) {
-#pragma unroll
-  for (int np = 0; np < 4; np++) {
-    const int row = 16 * np + 8 * (lane >> 4) + (lane & 7), chunk = 2 * kt + ((lane >> 3) & 1);
-    uint32_t b[4];
-    ldsm_x4(b, &tab[row][swz(row, chunk)]);
-    mma_bf16(acc[2 * np], a, b[0], b[1]);
-    mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
-  }
-}
+// ---------------------------------------------------------------------------
+// Coding: logits on the tensor cores (tcgen05, tensor memory)
 
-// bf16 1.0 at the element of value v among the pair (base, base + 1).
-__device__ __forceinline__ uint32_t onehot2(int v, int base) {
-  return v == base ? 0x00003f80u : v == base + 1 ? 0x3f800000u : 0u;
-}
-
-// The warp's 64 rows per step: row lane is symbol s of the lane's node, row
-// 32 + lane symbol s + 128; tile m holds rows 16 m .. 16 m + 15, and lane
-// (g, t) = (lane / 4, lane % 4) holds rows 16 m + g and 16 m + g + 8 of each
-// tile, that is the nodes of lanes 16 (m & 1) + 8 h + g (h = 0, 1), and
-// columns 8 n + 2 t + e (e = 0, 1) of each n-tile.  lm_nodefrag is the node
-// sums at those places (constant over a node's 128 steps).
-struct lm_nodefrag {
-  float v[2][2][8][2];   // [m & 1][h][n][e]
+// Tables of a coding CTA, from a base of 1,024 bytes.  The B operands are
+// K-major rows of 64 bf16 in the 128-byte swizzle (chunk c of row j at
+// c ^ (j & 7)): w1t row k holds W1[72 ..][k] / 16, w2t row i holds W2[..][j] of
+// the unit j that accumulator column i is, lm_unit(i).
+struct lm_coder {
+  uint4 w1t[kLmHidden][8];
+  uint4 w2t[kLmHidden][8];
+  uint2 near[256];            // per symbol: its 8 neighbours, a byte each
+  float b1[kLmHidden];
+  uint64_t mbar;
+  uint32_t tmem;
+  int32_t stream[2];
+  uint32_t other[2][32];      // what the second warp of a pair hands to the first
 };
 
-// Chunk kc (hidden units 16 kc .. 16 kc + 15) of the lane's own node sums,
-// own[i] for unit 16 kc + i, spread to the warp's fragment places.
-__device__ __forceinline__ void lm_node_frag(const float* own, int kc, int lane, lm_nodefrag& F) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int i = 0; i < 16; i++) {
-    const int k = 16 * kc + i;
-#pragma unroll
-    for (int mm = 0; mm < 2; mm++)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const float x = __shfl_sync(0xffffffffu, own[i], 16 * mm + 8 * h + g);
-        if (((k >> 1) & 3) == t) F.v[mm][h][k >> 3][k & 1] = x;
-      }
+// Accumulator columns are ordered so that columns 2 i and 2 i + 1 belong to the
+// chains P_t and P_t+1 (t even) of layer 3: one packed operation serves both.
+__host__ __device__ __forceinline__ int lm_unit(int column) { return (column & ~7) + 2 * (column & 3) + (column >> 2 & 1); }
+
+// Layer 3 and the biases beside it, per pair of accumulator columns: a kernel
+// parameter, so that they are operands in constant memory (read from shared
+// memory, each by 32 lanes at once, they took as long as the arithmetic).
+struct lm_out_t {
+  struct { float b2[2], w3[3][2]; } at[kLmHidden / 2];
+  float b3[4];
+};
+static lm_out_t lm_out(const uint8_t* model) {
+  auto w = [&](int i) {
+    const uint8_t* p = model + kLmModelHeader + 2 * i;
+    return bf16_value(uint16_t(p[0] | p[1] << 8));
+  };
+  lm_out_t O = {};
+  for (int i = 0; i < kLmHidden; i++) {
+    O.at[i >> 1].b2[i & 1] = w(kLmB2 + lm_unit(i));
+    for (int c = 0; c < 3; c++) O.at[i >> 1].w3[c][i & 1] = w(kLmW3 + lm_unit(i) * kLmOut + c);
   }
+  for (int c = 0; c < 3; c++) O.b3[c] = w(kLmB3 + c);
+  return O;
 }
 
-// Logits of the two symbols of step s (rotations s and s + 128) of every
-// lane's node.  ctx[0], ctx[1] are the lane's contexts of the two symbols:
-// 4 bits u_q = v_2q + 4 v_2q+1 per quadrant q (bits 0-15), the previous
-// node's symbol (bits 16-17).  Layer 1's rotation, neighbour and
-// previous-node rows and layer 2 run on the tensor cores; layer 1's results
-// stay in registers as layer 2's A operand.
-__device__ __forceinline__ void lm_step_logits(const lm_tables& S, const lm_nodefrag& N, int lane, int s,
-                                               const uint32_t* ctx, float* zA, float* zB) {
-  const int g = lane >> 2, t = lane & 3;
-  uint32_t cx[2][2][2];   // [m & 1][h][symbol]
-#pragma unroll
-  for (int mm = 0; mm < 2; mm++)
-#pragma unroll
-    for (int h = 0; h < 2; h++)
-#pragma unroll
-      for (int sb = 0; sb < 2; sb++) cx[mm][h][sb] = __shfl_sync(0xffffffffu, ctx[sb], 16 * mm + 8 * h + g);
-  // Row lane is in tile lane / 16 (symbol s) and tile 2 + lane / 16 (s + 128),
-  // half (lane / 8) & 1 of quad lane & 7.
-  const int src = 4 * (lane & 7), mine = lane >> 4, half = (lane >> 3) & 1;
-  // Tile m = 2 sb + mm: one tile at a time (the loop over sb is not unrolled,
-  // so the tiles' registers are not live together)
-#pragma unroll
-  for (int mm = 0; mm < 2; mm++) {
-#pragma unroll 1
-    for (int sb = 0; sb < 2; sb++) {
-      const int r = s + 128 * sb;
-      // Layer 1 A operand: one-hot features.  k-tile 0 is the rotation
-      // (feature 4 q + i_q; the lane's columns 2 t, 2 t + 1 and 8 + 2 t,
-      // 9 + 2 t are quadrants t / 2 and 2 + t / 2), the same for every node;
-      // k-tiles 1 and 2 are neighbours n = 4 (kt - 1) + t / 2 and n + 2;
-      // k-tile 3 is the previous node's symbol (columns 0-3: lanes t < 2).
-      const int base = 2 * (t & 1);
-      uint32_t a1[4][4];
-      a1[0][0] = a1[0][1] = onehot2((r >> (2 * (t >> 1))) & 3, base);
-      a1[0][2] = a1[0][3] = onehot2((r >> (2 * (2 + (t >> 1)))) & 3, base);
-#pragma unroll
+__device__ void lm_build_coder(lm_coder& S, const uint16_t* __restrict__ P, int tid, int nt) {
+  auto w = [&](int i) { return bf16_value(P[i]); };
+  for (int i = tid; i < kLmHidden * 8; i += nt) {
+    const int j = i >> 3, c = i & 7, unit = lm_unit(j);
+    uint32_t v[4], u[4];
+    for (int e = 0; e < 4; e++) {
+      const int f = 8 * c + 2 * e;   // feature rows 72 + f, 72 + f + 1 (zero past the 52)
+      u[e] = v[e] = 0;
       for (int h = 0; h < 2; h++) {
-        const uint32_t u = sb ? cx[mm][h][1] : cx[mm][h][0];
-#pragma unroll
-        for (int kt = 1; kt < 3; kt++) {
-          const int n0 = 4 * (kt - 1) + (t >> 1);
-          a1[kt][h] = onehot2(int(u >> (2 * n0)) & 3, base);
-          a1[kt][2 + h] = onehot2(int(u >> (2 * (n0 + 2))) & 3, base);
-        }
-        a1[3][h] = t < 2 ? onehot2(int(u >> 16) & 3, 2 * t) : 0u;
-        a1[3][2 + h] = 0u;
-      }
-      float acc[8][4];
-#pragma unroll
-      for (int n = 0; n < 8; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-#pragma unroll
-      for (int kt = 0; kt < 4; kt++) mma_row(acc, a1[kt], S.w1t, kt, lane);
-      // a1 = node + S1, quantized: n-tiles 2 k and 2 k + 1 of layer 1 are the
-      // k-tile k of layer 2's A operand
-      uint32_t a2[4][4];
-#pragma unroll
-      for (int n = 0; n < 8; n++) {
-        const float q00 = lm_act_q(f_add(N.v[mm][0][n][0], acc[n][0]));
-        const float q01 = lm_act_q(f_add(N.v[mm][0][n][1], acc[n][1]));
-        const float q10 = lm_act_q(f_add(N.v[mm][1][n][0], acc[n][2]));
-        const float q11 = lm_act_q(f_add(N.v[mm][1][n][1], acc[n][3]));
-        a2[n >> 1][2 * (n & 1)] = __byte_perm(f_raw(q00), f_raw(q01), 0x7632);
-        a2[n >> 1][2 * (n & 1) + 1] = __byte_perm(f_raw(q10), f_raw(q11), 0x7632);
-      }
-#pragma unroll
-      for (int n = 0; n < 8; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-#pragma unroll
-      for (int kt = 0; kt < 4; kt++) mma_row(acc, a2[kt], S.w2t, kt, lane);
-      // Layer 3 on the accumulators: the lane's columns make its P_t
-      float p0[3] = {0.f, 0.f, 0.f}, p1[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-      for (int n = 0; n < 8; n++)
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const int j = 8 * n + 2 * t + e;
-          const float4 w3 = *reinterpret_cast<const float4*>(S.w3[j]);
-          const float b2 = S.b2[j];
-          const float h0 = relu(f_fma(acc[n][e], kLmActInv, b2)), h1 = relu(f_fma(acc[n][2 + e], kLmActInv, b2));
-          p0[0] = f_fma(w3.x, h0, p0[0]);
-          p0[1] = f_fma(w3.y, h0, p0[1]);
-          p0[2] = f_fma(w3.z, h0, p0[2]);
-          p1[0] = f_fma(w3.x, h1, p1[0]);
-          p1[1] = f_fma(w3.y, h1, p1[1]);
-          p1[2] = f_fma(w3.z, h1, p1[2]);
-        }
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        // (P0 + P1) + (P2 + P3); addition commutes, so every lane of the
-        // quad ends with the same bits; then to the row's own lane
-        float q0 = f_add(p0[c], __shfl_xor_sync(0xffffffffu, p0[c], 1));
-        float q1 = f_add(p1[c], __shfl_xor_sync(0xffffffffu, p1[c], 1));
-        q0 = f_add(S.b3[c], f_add(q0, __shfl_xor_sync(0xffffffffu, q0, 2)));
-        q1 = f_add(S.b3[c], f_add(q1, __shfl_xor_sync(0xffffffffu, q1, 2)));
-        const float v0 = __shfl_sync(0xffffffffu, q0, src), v1 = __shfl_sync(0xffffffffu, q1, src);
-        if (mm == mine) {
-          const float v = half ? v1 : v0;
-          if (sb) zB[c] = v;
-          else zA[c] = v;
-        }
+        // the sixteenth of a bf16 is one, except below 2^-122, where nothing is left of it in an activation
+        if (f + h < kLmCtxRows)
+          u[e] |= uint32_t(bf16_round(f_mul(w(kLmW1 + (kLmRot + f + h) * kLmHidden + j), kLmActInv))) << (16 * h);
+        v[e] |= uint32_t(P[kLmW2 + (f + h) * kLmHidden + unit]) << (16 * h);
       }
     }
+    S.w1t[j][swz(j, c)] = make_uint4(u[0], u[1], u[2], u[3]);
+    S.w2t[j][swz(j, c)] = make_uint4(v[0], v[1], v[2], v[3]);
   }
+  for (int r = tid; r < 256; r += nt) {
+    uint32_t at[2] = {0, 0};
+    for (int n = 0; n < 8; n++) at[n >> 2] |= uint32_t(lm_neighbour(r, n)) << (8 * (n & 3));
+    S.near[r] = make_uint2(at[0], at[1]);
+  }
+  for (int i = tid; i < kLmHidden; i += nt) S.b1[i] = w(kLmB1 + i);
+  // (read by the tensor cores)
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// Tensor memory of a CTA, by column: the accumulators of its 128 rows, then
+// the A operand (two bf16 to a column); a warp reads and writes its 32 lanes.
+constexpr uint32_t kLmTmemCols = 128, kLmAcc = 0, kLmOperand = 64;
+// Instruction descriptor: fp32 accumulators, bf16 A and B, both K-major, N = 64, M = 128.
+constexpr uint32_t kLmIdesc = 1u << 4 | 1u << 7 | 1u << 10 | (kLmHidden / 8) << 17 | (128 / 16) << 24;
+
+// Shared-memory descriptor of a table: 128-byte swizzle, groups of 8 rows 1,024 bytes apart.
+__device__ __forceinline__ uint64_t lm_desc(const void* table) {
+  const uint64_t a = __cvta_generic_to_shared(table);
+  return (a >> 4) | uint64_t(1) << 16 | uint64_t(1024 >> 4) << 32 | uint64_t(1) << 46 | uint64_t(2) << 61;
+}
+// accumulators = operand x table (K = 64, in steps of 16), then an arrival on the barrier; one thread.
+__device__ __forceinline__ void lm_product(lm_coder& S, const void* table) {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint64_t desc = lm_desc(table);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+                 :: "r"(S.tmem + kLmAcc), "r"(S.tmem + kLmOperand + 8 * k), "l"(desc + 2 * k), "r"(kLmIdesc),
+                    "r"(uint32_t(k > 0)) : "memory");
+  }
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+               :: "r"(unsigned(__cvta_generic_to_shared(&S.mbar))) : "memory");
+}
+// Waits for a product; false if it has not come after a bounded number of polls.
+__device__ __forceinline__ bool lm_product_wait(lm_coder& S, uint32_t& phase) {
+  const unsigned bar = unsigned(__cvta_generic_to_shared(&S.mbar));
+  uint32_t done = 0;
+  for (int poll = 0; poll < (1 << 20) && !done; poll++)
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n"
+                 : "=r"(done) : "r"(bar), "r"(phase) : "memory");
+  phase ^= 1;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return done != 0;
+}
+
+#define PG_R8(v, b) "r"(v[b]), "r"(v[b + 1]), "r"(v[b + 2]), "r"(v[b + 3]), "r"(v[b + 4]), "r"(v[b + 5]), "r"(v[b + 6]), "r"(v[b + 7])
+#define PG_W8(v, b) "=r"(v[b]), "=r"(v[b + 1]), "=r"(v[b + 2]), "=r"(v[b + 3]), "=r"(v[b + 4]), "=r"(v[b + 5]), "=r"(v[b + 6]), "=r"(v[b + 7])
+// 32 columns of the thread's row (the wait belongs to the load: nothing may use the registers before it).
+__device__ __forceinline__ void tmem_ld(uint32_t* v, uint32_t at) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+               "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
+               "tcgen05.wait::ld.sync.aligned;\n"
+               : PG_W8(v, 0), PG_W8(v, 8), PG_W8(v, 16), PG_W8(v, 24) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t at, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+               "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
+               :: "r"(at), PG_R8(v, 0), PG_R8(v, 8), PG_R8(v, 16), PG_R8(v, 24) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t at, const uint32_t* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
+               :: "r"(at), PG_R8(v, 0) : "memory");
+}
+#undef PG_R8
+#undef PG_W8
+__device__ __forceinline__ void tmem_stored() {
+  asm volatile("tcgen05.wait::st.sync.aligned;\ntcgen05.fence::before_thread_sync;\n" ::: "memory");
+}
+
+// Two fp32 operations, each rounded as usual, in one instruction.
+__device__ __forceinline__ uint64_t f2(float a, float b) { return uint64_t(f_raw(b)) << 32 | f_raw(a); }
+__device__ __forceinline__ float f2_lo(uint64_t v) { return f_bits(uint32_t(v)); }
+__device__ __forceinline__ float f2_hi(uint64_t v) { return f_bits(uint32_t(v >> 32)); }
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ float f_add_sat(float a, float b) {   // to [0, 1]; 0 for NaN
+  float d;
+  asm("add.rn.sat.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ uint32_t shl_clamped(uint32_t v, uint32_t by) {   // 0 from 32 on
+  uint32_t d;
+  asm("shl.b32 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(by));
+  return d;
+}
+// bf16 1.0 at element v16 / 16 of four: two words of the A operand.
+__device__ __forceinline__ void onehot4(uint32_t* op, uint32_t v16) {
+  op[0] = shl_clamped(0x3f80u, v16);
+  op[1] = shl_clamped(0x3f80u, v16 - 32u);
+}
+
+// lm_act_q of two sums, as a bf16 pair.  a, b are the node's sums and s, t
+// layer 1's products, all a sixteenth of theirs (exact), so that one
+// saturated addition is the sum held to [0, 1], a 256th of the activation,
+// with the cut at 256: adding 2^23 rounds it to an integer, and what then is
+// 256 becomes 255.
+__device__ __forceinline__ uint32_t lm_act_q2(float a, float s, float b, float t) {
+  constexpr float two23 = 8388608.f;
+  const uint64_t y = f2(f_add_sat(a, s), f_add_sat(b, t));
+  const uint64_t q = f2_add(f2_fma(y, f2(256.f, 256.f), f2(two23, two23)), f2(-two23, -two23));
+  uint32_t d;
+  asm("min.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(__byte_perm(uint32_t(q), uint32_t(q >> 32), 0x7632)), "r"(0x437f437fu));
+  return d;
+}
+
+// Frequencies of symbol r of the thread's node, given the symbols coded
+// before it: row has 16 v per symbol, 48 for those not coded yet (like a value of
+// 3), prev the previous node's; node: the node's sums / 16.  The CTA's 128
+// threads are the 128 rows of the products and come here together.  Returns
+// false for all of them if a product did not come.
+constexpr int kLmChunk = 32;   // accumulator columns read at a time
+__device__ __forceinline__ bool lm_step_freqs(lm_coder& S, const lm_out_t& O, const uint8_t* row, const uint8_t* prev,
+                                              int r, const float* node, uint32_t& phase, bool& ok, lm_freq_t& F) {
+  const uint32_t tm = S.tmem + (threadIdx.x >> 5 << 21);   // the warp's lanes
+  {
+    uint32_t op[32];
+#pragma unroll
+    for (int q = 0; q < 4; q++) onehot4(op + 2 * q, uint32_t(r >> (2 * q) & 3) << 4);
+    const uint2 at = S.near[r];
+#pragma unroll
+    for (int n = 0; n < 8; n++) onehot4(op + 8 + 2 * n, row[(n < 4 ? at.x : at.y) >> (8 * (n & 3)) & 255]);
+    onehot4(op + 24, prev[r]);
+#pragma unroll
+    for (int i = 26; i < 32; i++) op[i] = 0;
+    tmem_st32(tm + kLmOperand, op);
+  }
+  tmem_stored();
+  if (__syncthreads_or(!ok)) return false;
+  if (threadIdx.x == 0) lm_product(S, S.w1t);
+  ok &= lm_product_wait(S, phase);
+#pragma unroll
+  for (int h = 0; h < kLmHidden; h += kLmChunk) {
+    uint32_t acc[kLmChunk], op[kLmChunk / 2];
+    tmem_ld(acc, tm + kLmAcc + h);
+#pragma unroll
+    for (int i = 0; i < kLmChunk / 2; i++)
+      op[i] = lm_act_q2(node[h + 2 * i], f_bits(acc[2 * i]), node[h + 2 * i + 1], f_bits(acc[2 * i + 1]));
+#pragma unroll
+    for (int i = 0; i < kLmChunk / 2; i += 8) tmem_st8(tm + kLmOperand + h / 2 + i, op + i);
+  }
+  tmem_stored();
+  if (__syncthreads_or(!ok)) return false;
+  if (threadIdx.x == 0) lm_product(S, S.w2t);
+  ok &= lm_product_wait(S, phase);
+  uint64_t part[2][3] = {};   // P_0 and P_1, P_2 and P_3
+#pragma unroll
+  for (int h = 0; h < kLmHidden; h += kLmChunk) {
+    uint32_t acc[kLmChunk];
+    tmem_ld(acc, tm + kLmAcc + h);
+#pragma unroll
+    for (int i = 0; i < kLmChunk / 2; i++) {
+      const auto& o = O.at[h / 2 + i];
+      const uint64_t a = f2_fma(uint64_t(acc[2 * i + 1]) << 32 | acc[2 * i], f2(kLmActInv, kLmActInv), f2(o.b2[0], o.b2[1]));
+      const uint64_t v = f2(relu(f2_lo(a)), relu(f2_hi(a)));
+#pragma unroll
+      for (int c = 0; c < 3; c++) part[i & 1][c] = f2_fma(f2(o.w3[c][0], o.w3[c][1]), v, part[i & 1][c]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  float z[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    z[c] = f_add(O.b3[c], f_add(f_add(f2_lo(part[0][c]), f2_hi(part[0][c])), f_add(f2_lo(part[1][c]), f2_hi(part[1][c]))));
+  F = lm_freqs(z);
+  return true;
 }
 
 // Neighbour context of symbol r from the node's symbols (those of earlier
@@ -329,51 +418,6 @@ __device__ __forceinline__ int lm_load_node(const lm_block_t& B, int64_t i, cons
   return lm_node_features(qid, T.unpack, feats);
 }
 
-// The lane's node: its node sums (b1 + stone rows ascending), 16 units at a
-// time, spread to the warp's fragment places.
-__device__ __forceinline__ void lm_round_nodes(const lm_tables& S, const uint16_t* __restrict__ P,
-                                               const lm_block_t& B, int64_t i, bool active, const dev_tables_t& T,
-                                               int lane, lm_nodefrag& N) {
-  uint8_t feats[36];
-  const int nf = active ? lm_load_node(B, i, T, feats) : 0;
-#pragma unroll
-  for (int kc = 0; kc < 4; kc++) {
-    float own[16];
-#pragma unroll
-    for (int u = 0; u < 16; u++) own[u] = S.b1[16 * kc + u];
-    for (int f = 0; f < nf; f++) {
-      const uint4* row = reinterpret_cast<const uint4*>(P + kLmW1 + feats[f] * kLmHidden + 16 * kc);
-#pragma unroll
-      for (int c = 0; c < 2; c++) {
-        const uint4 v = ldg(row + c);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          own[8 * c + 2 * e] = f_add(own[8 * c + 2 * e], f_bits(w[e] << 16));
-          own[8 * c + 2 * e + 1] = f_add(own[8 * c + 2 * e + 1], f_bits(w[e] & 0xffff0000u));
-        }
-      }
-    }
-    lm_node_frag(own, kc, lane, N);
-  }
-}
-
-// A run's previous node (its symbols, 2 bits each, 17 words a lane so that
-// lanes reading the same rotation use different banks); 3 for every
-// rotation before a run's first node.
-constexpr int kLmPrevWords = 17;
-__device__ __forceinline__ int lm_prev_sym(const uint32_t* prev, int r) { return int(prev[r >> 4] >> (2 * (r & 15))) & 3; }
-__device__ __forceinline__ void lm_prev_none(uint32_t* prev) {
-  for (int w = 0; w < 16; w++) prev[w] = 0xffffffffu;
-}
-__device__ __forceinline__ void lm_prev_from(uint32_t* prev, const uint8_t* sym) {
-  for (int w = 0; w < 16; w++) {
-    uint32_t v = 0;
-    for (int k = 0; k < 16; k++) v |= uint32_t(sym[16 * w + k] & 3) << (2 * k);
-    prev[w] = v;
-  }
-}
-
 __device__ __forceinline__ void put16(uint8_t* p, uint16_t v) { p[0] = uint8_t(v); p[1] = uint8_t(v >> 8); }
 __device__ __forceinline__ uint16_t get16(const uint8_t* p) { return uint16_t(p[0] | p[1] << 8); }
 __device__ __forceinline__ void put32(uint8_t* p, uint32_t v) { for (int i = 0; i < 4; i++) p[i] = uint8_t(v >> (8 * i)); }
@@ -381,66 +425,157 @@ __device__ __forceinline__ uint32_t get32(const uint8_t* p) {
   return uint32_t(p[0]) | uint32_t(p[1]) << 8 | uint32_t(p[2]) << 16 | uint32_t(p[3]) << 24;
 }
 
-// Dynamic shared memory of the coding kernels: the tables, then per warp its
-// lanes' nodes' symbols (one row of 256 bytes a lane, rows 260 bytes apart
-// so that lanes reading the same rotation use different banks), their
-// previous nodes' symbols (packed) and, for the decoder, a window of the
-// stream's next words.
+// The coding kernels give a stream two warps, which code the two symbols of a
+// step side by side (neither is the other's neighbour): lane l of both has
+// the node of the stream's lane l, the second warp hands its frequencies to
+// the first, and that one keeps the rANS states.  A CTA is two such pairs,
+// 128 rows for one product of the tensor cores.  All its warps take their
+// steps together; nodes have 128 steps, so the streams of a CTA begin
+// their nodes together, and a pair without a stream keeps step without
+// coding.
+//
+// Dynamic shared memory: the tables, then per pair two buffers of its nodes'
+// symbols (the nodes being coded and the ones before them; a row of 256 bytes
+// a lane, rows 260 bytes apart so that lanes reading the same rotation use
+// different banks) and, for the decoder, a window of the stream's next words.
+//
+// Bound by the chain of a step: 5,000 cycles with three CTAs an SM, of which
+// the products take 500 each (issue to arrival), layer 3 900, the frequencies 770, the states 900; its
+// instructions alone would take about 2,000.  2,048 blocks of a solved slice:
+// 166 ms each way with mma.sync (whose 256 products a step and stream were
+// most of it), 87 ms now.  Four CTAs of 128 registers: 100 ms.
 constexpr int kLmSymRow = 260;
-constexpr int kLmWordWin = 1024;   // the decoder's window of upcoming stream words, per warp
-constexpr size_t kLmWarpSmem = size_t(32) * kLmSymRow + size_t(32) * 4 * kLmPrevWords + 2 * kLmWordWin;
-constexpr size_t kLmCodeSmem = sizeof(lm_tables) + kLmWarpSmem * kLmWarps;
-static_assert(sizeof(lm_tables) % 16 == 0 && kLmWarpSmem % 16 == 0, "coding rows stay 16-byte aligned");
+constexpr int kLmWordWin = 1024;   // the decoder's window of upcoming stream words
+constexpr size_t kLmPairSmem = size_t(2) * 32 * kLmSymRow + 2 * kLmWordWin;
+constexpr size_t kLmCodeSmem = 1024 + sizeof(lm_coder) + 2 * kLmPairSmem;   // (from a multiple of 1,024)
+constexpr int kLmCodeCtas = 3;
+static_assert(sizeof(lm_coder) % 16 == 0 && kLmPairSmem % 16 == 0, "coding rows stay aligned");
+static_assert(kLmCodeCtas * kLmTmemCols <= 512, "tensor memory of an SM");
 
-// A node's 256 symbols between global memory and its shared-memory row.
-__device__ __forceinline__ int lm_row_in(uint8_t* row, const uint8_t* g) {
-  int bad = 0;
-  if ((reinterpret_cast<uintptr_t>(g) & 3) == 0) {
-    for (int w = 0; w < 64; w++) {
-      const uint32_t v = reinterpret_cast<const uint32_t*>(g)[w];
-      bad |= (v & 0xfcfcfcfcu) != 0 || (v & v >> 1 & 0x01010101u) != 0;   // a byte above 2
-      reinterpret_cast<uint32_t*>(row)[w] = v;
+struct lm_pair {   // a thread's place, and its pair's buffers
+  int pair, half, lane;
+  uint8_t* row[2];
+  uint16_t* win;
+  // (a barrier named by a register would reserve all 16 of the CTA's, and with them the SM's room for other CTAs)
+  __device__ __forceinline__ void sync() const {
+    if (pair) asm volatile("bar.sync 2, 64;" ::: "memory");
+    else asm volatile("bar.sync 1, 64;" ::: "memory");
+  }
+  // The pair's threads share a row's words, or its bytes
+  __device__ __forceinline__ void fill(uint8_t* to) const {
+    for (int w = half; w < 64; w += 2) reinterpret_cast<uint32_t*>(to)[w] = 0x30303030u;
+  }
+  // A node's 256 symbols between global memory and its row (16 v there); true if one is above 2.
+  __device__ __forceinline__ bool in(uint8_t* to, const uint8_t* g) const {
+    bool bad = false;
+    if ((reinterpret_cast<uintptr_t>(g) & 3) == 0) {
+#pragma unroll 8
+      for (int w = half; w < 64; w += 2) {
+        const uint32_t v = reinterpret_cast<const uint32_t*>(g)[w];
+        bad |= (v & 0xfcfcfcfcu) != 0 || (v & v >> 1 & 0x01010101u) != 0;   // a byte above 2
+        reinterpret_cast<uint32_t*>(to)[w] = (v & 0x03030303u) << 4;
+      }
+    } else {
+      for (int k = half; k < 256; k += 2) {
+        const uint8_t v = g[k];
+        bad |= v > 2;
+        to[k] = uint8_t((v & 3) << 4);
+      }
     }
-  } else {
-    for (int k = 0; k < 256; k++) {
-      const uint8_t v = g[k];
-      bad |= v > 2;
-      row[k] = v;
+    return bad;
+  }
+  __device__ __forceinline__ void out(const uint8_t* from, uint8_t* g) const {
+    if ((reinterpret_cast<uintptr_t>(g) & 3) == 0) {
+#pragma unroll 8
+      for (int w = half; w < 64; w += 2)
+        reinterpret_cast<uint32_t*>(g)[w] = reinterpret_cast<const uint32_t*>(from)[w] >> 4 & 0x03030303u;
+    } else {
+      for (int k = half; k < 256; k += 2) g[k] = uint8_t(from[k] >> 4);
     }
   }
-  return bad;
+  // The next stream of a launch, largest first (streams are handed out one at
+  // a time through a counter, in the order the host sorted them), or -1.
+  __device__ __forceinline__ int next_stream(lm_coder& S, int* next, const int32_t* order, int nstreams) const {
+    if (half == 0 && lane == 0) {
+      const int k = atomicAdd(next, 1);
+      S.stream[pair] = k < nstreams ? order[k] : -1;
+    }
+    sync();
+    const int s = S.stream[pair];
+    sync();
+    return s;
+  }
+};
+
+// Tables, tensor memory and barrier of a coding CTA; and giving them back.
+__device__ lm_coder& lm_coder_begin(unsigned char* raw, const uint16_t* __restrict__ P, lm_pair& W) {
+  unsigned char* base = raw + ((1024 - (__cvta_generic_to_shared(raw) & 1023)) & 1023);
+  lm_coder& S = *reinterpret_cast<lm_coder*>(base);
+  const int warp = threadIdx.x >> 5;
+  W.pair = warp >> 1;
+  W.half = warp & 1;
+  W.lane = threadIdx.x & 31;
+  unsigned char* mine = base + sizeof(lm_coder) + kLmPairSmem * W.pair;
+  for (int b = 0; b < 2; b++) W.row[b] = mine + (32 * b + W.lane) * kLmSymRow;
+  W.win = reinterpret_cast<uint16_t*>(mine + 2 * 32 * kLmSymRow);
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(unsigned(__cvta_generic_to_shared(&S.tmem))), "r"(kLmTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(unsigned(__cvta_generic_to_shared(&S.mbar))) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  lm_build_coder(S, P, threadIdx.x, blockDim.x);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  return S;
 }
-__device__ __forceinline__ void lm_row_out(const uint8_t* row, uint8_t* g) {
-  if ((reinterpret_cast<uintptr_t>(g) & 3) == 0) {
-    for (int w = 0; w < 64; w++) reinterpret_cast<uint32_t*>(g)[w] = reinterpret_cast<const uint32_t*>(row)[w];
-  } else {
-    for (int k = 0; k < 256; k++) g[k] = row[k];
-  }
+__device__ void lm_coder_end(lm_coder& S) {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (threadIdx.x < 32)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(S.tmem), "r"(kLmTmemCols) : "memory");
+}
+
+// The sums of the thread's node (b1 + stone rows ascending), / 16.
+__device__ __forceinline__ void lm_coder_node(const lm_coder& S, const uint16_t* __restrict__ P, const lm_block_t& B,
+                                              int64_t i, bool active, const dev_tables_t& T, float* node) {
+  uint8_t feats[36];
+  const int nf = active ? lm_load_node(B, i, T, feats) : 0;
+  lm_node_sum(S.b1, P, feats, nf, node);
+#pragma unroll
+  for (int k = 0; k < kLmHidden; k++) node[k] = f_mul(node[k], kLmActInv);
 }
 
 // Append one 16-bit word per renormalizing lane, in lane order (encoder).
-__device__ __forceinline__ void lm_put_state(uint32_t& x, const lm_freq_t& F, int v, bool active, uint8_t* words,
+__device__ __forceinline__ void lm_put_state(uint32_t& x, uint32_t f, uint32_t cum, bool active, uint8_t* words,
                                              uint32_t& len, unsigned below) {
-  const bool emit = active && x >= (F.f[v] << 17);
+  const bool emit = active && x >= (f << 17);
   const unsigned mask = __ballot_sync(0xffffffffu, emit);
   if (emit) {
     put16(words + 2 * (len + __popc(mask & below)), uint16_t(x));
     x >>= 16;
   }
   len += __popc(mask);
-  if (active) x = ((x / F.f[v]) << kLmProbBits) + x % F.f[v] + F.cum[v];
+  if (active) x = ((x / f) << kLmProbBits) + x % f + cum;
 }
 
-// Decode one symbol per active lane and take this step's words (decoder).
-// Words [wlo, wlo + kLmWordWin) are also in win.
-__device__ __forceinline__ int lm_get_symbol(uint32_t& x, const lm_freq_t& F, bool active, const uint8_t* words,
+// Decode one symbol per active lane and take this step's words (decoder);
+// f0 and f1 are the frequencies of symbols 0 and 1.  Words [wlo, wlo +
+// kLmWordWin) are also in win.
+__device__ __forceinline__ int lm_get_symbol(uint32_t& x, uint32_t f0, uint32_t f1, bool active, const uint8_t* words,
                                              const uint16_t* win, int64_t wlo, int64_t& ptr, unsigned above,
                                              int& bad) {
   int v = 0;
   if (active) {
-    const uint32_t slot = x & (kLmProbTotal - 1);
-    v = slot < F.cum[1] ? 0 : slot < F.cum[2] ? 1 : 2;
-    x = F.f[v] * (x >> kLmProbBits) + slot - F.cum[v];
+    const uint32_t slot = x & (kLmProbTotal - 1), f01 = f0 + f1;
+    v = slot < f0 ? 0 : slot < f01 ? 1 : 2;
+    const uint32_t cum = v == 0 ? 0 : v == 1 ? f0 : f01, f = v == 0 ? f0 : v == 1 ? f1 : kLmProbTotal - f01;
+    x = f * (x >> kLmProbBits) + slot - cum;
   }
   const bool need = active && x < kLmLower;
   const unsigned mask = __ballot_sync(0xffffffffu, need);
@@ -454,90 +589,100 @@ __device__ __forceinline__ int lm_get_symbol(uint32_t& x, const lm_freq_t& F, bo
   return v;
 }
 
-// The next stream of a launch, largest first: streams are handed to warps
-// one at a time through a counter, in the order the host sorted them.
-__device__ __forceinline__ int lm_next_stream(int* next, const int32_t* order, int nstreams, int lane) {
-  int k = 0;
-  if (lane == 0) k = atomicAdd(next, 1);
-  k = __shfl_sync(0xffffffffu, k, 0);
-  return k < nstreams ? order[k] : -1;
-}
-
-// One warp per stream (grid-stride over streams).  sizes[s] = stream bytes, or
-// PG_ERR_ARG for a symbol above 2 or a symbol count that does not match.
-// Coding kernels are compiled for three CTAs (12 warps) per SM.
-constexpr int kLmCodeCtas = 3;
-
+// sizes[s] = stream bytes, or PG_ERR_ARG for a symbol above 2 or a symbol
+// count that does not match.
 __global__ void __launch_bounds__(kLmThreads, kLmCodeCtas)
 lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t* __restrict__ blocks, int nstreams,
                  const int32_t* __restrict__ order, int* __restrict__ next, const uint8_t* __restrict__ symbols,
                  const int64_t* __restrict__ offsets, uint8_t* __restrict__ out,
-                 const int64_t* __restrict__ out_offsets, int64_t* __restrict__ sizes, const dev_tables_t T) {
+                 const int64_t* __restrict__ out_offsets, int64_t* __restrict__ sizes, const dev_tables_t T,
+                 const __grid_constant__ lm_out_t O) {
   extern __shared__ __align__(16) unsigned char lm_smem_raw[];
-  lm_tables& S = *reinterpret_cast<lm_tables*>(lm_smem_raw);
-  lm_build_tables(S, P, threadIdx.x, blockDim.x);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint8_t* row = lm_smem_raw + sizeof(lm_tables) + kLmWarpSmem * warp + kLmSymRow * lane;
-  uint32_t* prev = reinterpret_cast<uint32_t*>(lm_smem_raw + sizeof(lm_tables) + kLmWarpSmem * warp +
-                                               32 * kLmSymRow) + kLmPrevWords * lane;
-  const unsigned below = (1u << lane) - 1;
-  for (int s; (s = lm_next_stream(next, order, nstreams, lane)) >= 0;) {
-    const lm_block_t B = blocks[s];
-    const int64_t n = B.nodes;
-    uint8_t* base = out + out_offsets[s];
-    if (offsets[s + 1] - offsets[s] != 256 * n) {
-      if (lane == 0) sizes[s] = PG_ERR_ARG;
-      continue;
+  lm_pair W;
+  lm_coder& S = lm_coder_begin(lm_smem_raw, P, W);
+  const unsigned below = (1u << W.lane) - 1;
+  int s = -1, cur = 0;
+  bool more = true, ok = true, whole = true;
+  uint32_t phase = 0;
+  int64_t n = 0, R = 0, round = -1;   // R: the run of nodes of each lane
+  const uint8_t* sym0 = nullptr;
+  uint8_t *base = nullptr, *words = nullptr;
+  uint32_t x = kLmLower, len = 0;
+  int bad = 0;
+  lm_block_t B = {};
+  while (whole) {
+    while (more && round < 0) {
+      if (s >= 0) {   // the stream is done
+        if (W.half) S.other[W.pair][W.lane] = uint32_t(bad);
+        W.sync();
+        if (!W.half) {
+          put32(base + 20 + 4 * W.lane, x);
+          bad = __any_sync(0xffffffffu, bad | int(S.other[W.pair][W.lane]));
+          if (W.lane == 0) {
+            put32(base, kLmVersion);
+            put32(base + 4, uint32_t(hash));
+            put32(base + 8, uint32_t(hash >> 32));
+            put32(base + 12, uint32_t(n));
+            put32(base + 16, len);
+            sizes[s] = bad ? PG_ERR_ARG : kLmStreamHeader + 2 * int64_t(len);
+          }
+        }
+      }
+      s = W.next_stream(S, next, order, nstreams);
+      more = s >= 0;
+      if (!more) break;
+      B = blocks[s];
+      n = B.nodes;
+      if (offsets[s + 1] - offsets[s] != 256 * n) {
+        if (W.half == 0 && W.lane == 0) sizes[s] = PG_ERR_ARG;
+        s = -1;
+        continue;
+      }
+      sym0 = symbols + offsets[s];
+      base = out + out_offsets[s];
+      words = base + kLmStreamHeader;
+      x = kLmLower;
+      len = 0;
+      bad = 0;
+      R = (n + 31) / 32;
+      round = R - 1;
+      const int64_t i = R * W.lane + round;
+      if (i < n) bad |= W.in(W.row[cur], sym0 + 256 * i);
     }
-    const uint8_t* sym0 = symbols + offsets[s];
-    uint8_t* words = base + kLmStreamHeader;
-    uint32_t x = kLmLower;
-    uint32_t len = 0;
-    int bad = 0;
-    const int64_t R = (n + 31) / 32;   // the run of nodes of each lane
-    for (int64_t round = R - 1; round >= 0; round--) {
-      const int64_t i = R * lane + round;
-      const bool active = i < n;
-      lm_nodefrag N;
-      lm_round_nodes(S, P, B, i, active, T, lane, N);
-      if (active) bad |= lm_row_in(row, sym0 + 256 * i);
-      if (active && round > 0) lm_prev_from(prev, sym0 + 256 * (i - 1));
-      else lm_prev_none(prev);
-      for (int st = 127; st >= 0; st--) {
-        uint32_t ctx[2] = {0u, 0u};
-        if (active) {
-          ctx[0] = lm_context_packed(row, st) | uint32_t(lm_prev_sym(prev, st)) << 16;
-          ctx[1] = lm_context_packed(row, st + 128) | uint32_t(lm_prev_sym(prev, st + 128)) << 16;
-        }
-        float zA[3], zB[3];
-        lm_step_logits(S, N, lane, st, ctx, zA, zB);
-        lm_freq_t FA = {}, FB = {};
-        int vA = 0, vB = 0;
-        if (active) {
-          FA = lm_freqs(zA);
-          FB = lm_freqs(zB);
-          vA = row[st] & 3;
-          vB = row[st + 128] & 3;
-          if (vA > 2) vA = 0;   // (flagged when the row was read)
-          if (vB > 2) vB = 0;
-        }
+    if (!__syncthreads_or(more)) break;
+    const int64_t i = R * W.lane + round;
+    const bool active = more && i < n;
+    float node[kLmHidden];
+    lm_coder_node(S, P, B, i, active, T, node);
+    uint8_t* row = W.row[cur];
+    const uint8_t* prev = W.row[cur ^ 1];
+    if (more) {
+      if (round == 0) W.fill(W.row[cur ^ 1]);
+      else if (i - 1 < n) bad |= W.in(W.row[cur ^ 1], sym0 + 256 * (i - 1));
+      W.sync();
+    }
+    for (int st = 127; st >= 0; st--) {
+      const int r = st + 128 * W.half;
+      lm_freq_t F;
+      whole = lm_step_freqs(S, O, row, prev, r, node, phase, ok, F);
+      if (!whole) break;
+      const int v = row[r] >> 4;
+      row[r] = 48;   // to the earlier steps' symbols, one that is not coded yet
+      uint32_t f = v == 1 ? F.f[1] : v == 2 ? F.f[2] : F.f[0], cum = v == 1 ? F.cum[1] : v == 2 ? F.cum[2] : 0u;
+      if (W.half) S.other[W.pair][W.lane] = f | cum << 16;
+      W.sync();
+      if (!W.half) {
         // the decoder takes s then s + 128, so the encoder puts s + 128 first
-        lm_put_state(x, FB, vB, active, words, len, below);
-        lm_put_state(x, FA, vA, active, words, len, below);
+        const uint32_t o = S.other[W.pair][W.lane];
+        lm_put_state(x, o & 0xffff, o >> 16, active, words, len, below);
+        lm_put_state(x, f, cum, active, words, len, below);
       }
     }
-    put32(base + 20 + 4 * lane, x);
-    bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) {
-      put32(base, kLmVersion);
-      put32(base + 4, uint32_t(hash));
-      put32(base + 8, uint32_t(hash >> 32));
-      put32(base + 12, uint32_t(n));
-      put32(base + 16, len);
-      sizes[s] = bad ? PG_ERR_ARG : kLmStreamHeader + 2 * int64_t(len);
-    }
+    cur ^= 1;
+    round--;
   }
+  if (!whole && s >= 0 && W.half == 0 && W.lane == 0) sizes[s] = PG_ERR_CUDA;
+  lm_coder_end(S);
 }
 
 // status[s] = symbols decoded, or PG_ERR_FORMAT / PG_ERR_CAPACITY.  Version-2
@@ -549,83 +694,99 @@ lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
                  const int64_t* __restrict__ in_offsets,
                  const int64_t* __restrict__ in_sizes, uint8_t* __restrict__ symbols,
                  const int64_t* __restrict__ sym_offsets, const int64_t* __restrict__ sym_caps,
-                 int64_t* __restrict__ status, const dev_tables_t T) {
+                 int64_t* __restrict__ status, const dev_tables_t T, const __grid_constant__ lm_out_t O) {
   extern __shared__ __align__(16) unsigned char lm_smem_raw[];
-  lm_tables& S = *reinterpret_cast<lm_tables*>(lm_smem_raw);
-  lm_build_tables(S, P, threadIdx.x, blockDim.x);
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint8_t* row = lm_smem_raw + sizeof(lm_tables) + kLmWarpSmem * warp + kLmSymRow * lane;
-  uint32_t* prev = reinterpret_cast<uint32_t*>(lm_smem_raw + sizeof(lm_tables) + kLmWarpSmem * warp +
-                                               32 * kLmSymRow) + kLmPrevWords * lane;
-  uint16_t* win = reinterpret_cast<uint16_t*>(lm_smem_raw + sizeof(lm_tables) + kLmWarpSmem * warp +
-                                              32 * kLmSymRow + 32 * 4 * kLmPrevWords);
-  const unsigned above = lane == 31 ? 0u : ~0u << (lane + 1);
-  for (int s; (s = lm_next_stream(next, order, nstreams, lane)) >= 0;) {
-    const lm_block_t B = blocks[s];
-    const int64_t n = B.nodes;
-    const uint8_t* base = in + in_offsets[s];
-    const int64_t size = in_sizes[s];
-    if (size < 4) continue;
-    const uint32_t version = get32(base);
-    if (version == 2) continue;
-    const uint64_t h = uint64_t(get32(base + 4)) | uint64_t(get32(base + 8)) << 32;
-    const uint32_t len = size >= kLmStreamHeader ? get32(base + 16) : 0;
-    if (version != kLmVersion || size < kLmStreamHeader || h != hash || get32(base + 12) != uint64_t(n) ||
-        int64_t(len) * 2 + kLmStreamHeader != size) {
-      if (lane == 0) status[s] = PG_ERR_FORMAT;
-      continue;
-    }
-    if (sym_caps[s] < 256 * n) {
-      if (lane == 0) status[s] = PG_ERR_CAPACITY;
-      continue;
-    }
-    const uint8_t* words = base + kLmStreamHeader;
-    uint8_t* out0 = symbols + sym_offsets[s];
-    uint32_t x = get32(base + 20 + 4 * lane);
-    int64_t ptr = len;  // words [0, ptr) are unread
-    int bad = 0;
-    const int64_t R = (n + 31) / 32;   // the run of nodes of each lane
-    for (int64_t round = 0; round < R; round++) {
-      const int64_t i = R * lane + round;
-      const bool active = i < n;
-      lm_nodefrag N;
-      lm_round_nodes(S, P, B, i, active, T, lane, N);
-      // the previous node of the run is the row of the last round
-      if (round > 0) lm_prev_from(prev, row);
-      else lm_prev_none(prev);
-      for (int w = 0; w < 64; w++) reinterpret_cast<uint32_t*>(row)[w] = 0u;
-      // the round's words are the last unread ones: stage up to kLmWordWin of them
-      const int64_t wlo = ptr > kLmWordWin ? ptr - kLmWordWin : 0;
-      __syncwarp();
-      for (int64_t w = wlo + lane; w < ptr; w += 32) win[w - wlo] = get16(words + 2 * w);
-      __syncwarp();
-      for (int st = 0; st < 128; st++) {
-        uint32_t ctx[2] = {0u, 0u};
-        if (active) {
-          ctx[0] = lm_context_packed(row, st) | uint32_t(lm_prev_sym(prev, st)) << 16;
-          ctx[1] = lm_context_packed(row, st + 128) | uint32_t(lm_prev_sym(prev, st + 128)) << 16;
-        }
-        float zA[3], zB[3];
-        lm_step_logits(S, N, lane, st, ctx, zA, zB);
-        lm_freq_t FA = {}, FB = {};
-        if (active) {
-          FA = lm_freqs(zA);
-          FB = lm_freqs(zB);
-        }
-        const int vA = lm_get_symbol(x, FA, active, words, win, wlo, ptr, above, bad);
-        const int vB = lm_get_symbol(x, FB, active, words, win, wlo, ptr, above, bad);
-        row[st] = uint8_t(vA);
-        row[st + 128] = uint8_t(vB);
+  lm_pair W;
+  lm_coder& S = lm_coder_begin(lm_smem_raw, P, W);
+  const bool first = W.half == 0 && W.lane == 0;
+  const unsigned above = W.lane == 31 ? 0u : ~0u << (W.lane + 1);
+  int s = -1, cur = 0;
+  bool more = true, ok = true, whole = true;
+  uint32_t phase = 0;
+  int64_t n = 0, R = 0, round = 0;   // R: the run of nodes of each lane
+  const uint8_t* words = nullptr;
+  uint8_t* out0 = nullptr;
+  uint32_t x = kLmLower;
+  int64_t ptr = 0;   // words [0, ptr) are unread
+  int bad = 0;
+  lm_block_t B = {};
+  while (whole) {
+    while (more && round == R) {
+      if (s >= 0 && !W.half) {
+        // A well-formed stream ends with every word read and every lane back
+        // at the encoder's initial state.
+        bad |= x != kLmLower;
+        bad = __any_sync(0xffffffffu, bad);
+        if (W.lane == 0) status[s] = (bad || ptr != 0) ? PG_ERR_FORMAT : 256 * n;
       }
-      if (active) lm_row_out(row, out0 + 256 * i);
+      s = W.next_stream(S, next, order, nstreams);
+      more = s >= 0;
+      if (!more) break;
+      const int now = s;
+      s = -1;   // (until the stream is known to be one to decode)
+      const uint8_t* base = in + in_offsets[now];
+      const int64_t size = in_sizes[now];
+      if (size < 4) continue;
+      const uint32_t version = get32(base);
+      if (version == 2) continue;
+      B = blocks[now];
+      n = B.nodes;
+      const uint64_t h = size >= kLmStreamHeader ? uint64_t(get32(base + 4)) | uint64_t(get32(base + 8)) << 32 : 0;
+      const uint32_t len = size >= kLmStreamHeader ? get32(base + 16) : 0;
+      if (version != kLmVersion || size < kLmStreamHeader || h != hash || get32(base + 12) != uint64_t(n) ||
+          int64_t(len) * 2 + kLmStreamHeader != size) {
+        if (first) status[now] = PG_ERR_FORMAT;
+        continue;
+      }
+      if (sym_caps[now] < 256 * n) {
+        if (first) status[now] = PG_ERR_CAPACITY;
+        continue;
+      }
+      s = now;
+      words = base + kLmStreamHeader;
+      out0 = symbols + sym_offsets[s];
+      x = get32(base + 20 + 4 * W.lane);
+      ptr = len;
+      bad = 0;
+      R = (n + 31) / 32;
+      round = 0;
+      W.fill(W.row[cur ^ 1]);
     }
-    // A well-formed stream ends with every word read and every lane back at
-    // the encoder's initial state.
-    bad |= x != kLmLower;
-    bad = __any_sync(0xffffffffu, bad);
-    if (lane == 0) status[s] = (bad || ptr != 0) ? PG_ERR_FORMAT : 256 * n;
+    if (!__syncthreads_or(more)) break;
+    const int64_t i = R * W.lane + round;
+    const bool active = more && i < n;
+    float node[kLmHidden];
+    lm_coder_node(S, P, B, i, active, T, node);
+    uint8_t* row = W.row[cur];
+    W.fill(row);
+    const uint8_t* prev = W.row[cur ^ 1];   // the previous node of the run is the row of the last round
+    // the round's words are the last unread ones: stage up to kLmWordWin of them
+    const int64_t wlo = ptr > kLmWordWin ? ptr - kLmWordWin : 0;
+    if (more && !W.half) {
+#pragma unroll 4
+      for (int64_t w = wlo + W.lane; w < ptr; w += 32) W.win[w - wlo] = get16(words + 2 * w);
+    }
+    if (more) W.sync();
+    for (int st = 0; st < 128; st++) {
+      const int r = st + 128 * W.half;
+      lm_freq_t F;
+      whole = lm_step_freqs(S, O, row, prev, r, node, phase, ok, F);
+      if (!whole) break;
+      if (W.half) S.other[W.pair][W.lane] = F.f[0] | F.f[1] << 16;
+      W.sync();
+      if (!W.half) {
+        const uint32_t o = S.other[W.pair][W.lane];
+        row[st] = uint8_t(lm_get_symbol(x, F.f[0], F.f[1], active, words, W.win, wlo, ptr, above, bad) << 4);
+        row[st + 128] = uint8_t(lm_get_symbol(x, o & 0xffff, o >> 16, active, words, W.win, wlo, ptr, above, bad) << 4);
+      }
+      W.sync();
+    }
+    if (active && whole) W.out(row, out0 + 256 * i);
+    cur ^= 1;
+    round++;
   }
+  if (!whole && s >= 0 && first) status[s] = PG_ERR_CUDA;
+  lm_coder_end(S);
 }
 
 // Frequencies of given samples (for checking the coding path against the CPU).
@@ -646,7 +807,7 @@ lm_freqs_kernel(const uint16_t* __restrict__ P, const lm_block_t* __restrict__ b
     uint8_t feats[36];
     const int nf = lm_load_node(blocks[s], i, T, feats);
     float node[kLmHidden];
-    lm_node_sum(S, P, feats, nf, node);
+    lm_node_sum(S.b1, P, feats, nf, node);
     int u[4];
     const uint8_t* sym = symbols + offsets[s] + 256 * i;
     lm_context_clamped(sym, r, u);
@@ -1261,14 +1422,14 @@ template<class K> static int lm_smem_opt_in(K kernel, size_t bytes) {
 }
 
 // The coding kernels: as many CTAs as are resident at once (the streams are
-// handed out dynamically), no more than there are streams for.
-template<class K> static int lm_code_grid(K kernel, int nstreams) {
-  int dev = 0, sms = 148, per = 1;
+// handed out dynamically), no more than there are streams for.  kLmCodeCtas
+// fit an SM by their launch bounds, shared and tensor memory; the occupancy
+// query answers 1 for any kernel that allocates tensor memory.
+static int lm_code_grid(int nstreams) {
+  int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kLmThreads, kLmCodeSmem) != cudaSuccess || per < 1)
-    per = 1;
-  return std::max(1, std::min((nstreams + kLmWarps - 1) / kLmWarps, per * sms));
+  return std::max(1, std::min((nstreams + 1) / 2, kLmCodeCtas * sms));
 }
 
 }  // namespace pg
@@ -1310,8 +1471,9 @@ extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t
   std::vector<lm_block_t> hb;
   if (int rc = lm_prepare(model, blocks, nstreams, st, L, &hb)) return rc;
   if (int rc = lm_smem_opt_in(lm_encode_kernel, kLmCodeSmem)) return rc;
-  lm_encode_kernel<<<lm_code_grid(lm_encode_kernel, nstreams), kLmThreads, kLmCodeSmem, st>>>(
-      L.params, L.hash, L.blocks, nstreams, L.order, L.next, symbols, offsets, out, out_offsets, sizes, *T);
+  lm_encode_kernel<<<lm_code_grid(nstreams), kLmThreads, kLmCodeSmem, st>>>(
+      L.params, L.hash, L.blocks, nstreams, L.order, L.next, symbols, offsets, out, out_offsets, sizes, *T,
+      lm_out(model));
   PG_CUDA(cudaGetLastError());
   // Format-2 streams of the same symbols; the smaller one is kept
   // alt_off[s] = slot of stream s; alt_off[nstreams + s] = its symbol count
@@ -1351,9 +1513,9 @@ extern "C" int pg_rans_learned_decode(const uint8_t* model, const pg_block_ref_t
   if (int rc = launch_rans_decode(in, in_offsets, in_sizes, nstreams, symbols, sym_offsets, sym_caps, status, 1, st))
     return rc;
   if (int rc = lm_smem_opt_in(lm_decode_kernel, kLmCodeSmem)) return rc;
-  lm_decode_kernel<<<lm_code_grid(lm_decode_kernel, nstreams), kLmThreads, kLmCodeSmem, st>>>(
+  lm_decode_kernel<<<lm_code_grid(nstreams), kLmThreads, kLmCodeSmem, st>>>(
       L.params, L.hash, L.blocks, nstreams, L.order, L.next, in, in_offsets, in_sizes, symbols, sym_offsets, sym_caps,
-      status, *T);
+      status, *T, lm_out(model));
   PG_CUDA(cudaGetLastError());
   return PG_OK;
 }

@@ -200,7 +200,14 @@ PG_HD void lm_grid_params(float* p) {
 // determinism matters, and every step is an exactly specified IEEE operation.
 PG_HD float lm_exp2(float d) {
   if (!(d >= -24.f)) return 0.f;
+  // (d plus 1.5 2^23, rounded down, has floor(d) in its last bits)
+#ifdef __CUDA_ARCH__
+  const float u = __fadd_rd(d, 12582912.f), n = f_add(u, -12582912.f);
+  const uint32_t scale = (f_raw(u) << 23) + 0x3f800000u;
+#else
   const float n = floorf(d);
+  const uint32_t scale = uint32_t(127 + int(n)) << 23;
+#endif
   const float t = f_add(d, -n);
   float p = 1.5252734e-05f;
   p = f_fma(p, t, 1.5403530e-04f);
@@ -210,7 +217,16 @@ PG_HD float lm_exp2(float d) {
   p = f_fma(p, t, 2.4022651e-01f);
   p = f_fma(p, t, 6.9314718e-01f);
   p = f_fma(p, t, 1.0f);
-  return f_mul(p, f_bits(uint32_t(127 + int(n)) << 23));
+  return f_mul(p, f_bits(scale));
+}
+
+// The integer part of q, 0 <= q < 2^22.
+PG_HD uint32_t lm_trunc(float q) {
+#ifdef __CUDA_ARCH__
+  return f_raw(__fadd_rd(q, 8388608.f)) & 0x7fffffu;
+#else
+  return uint32_t(q);
+#endif
 }
 
 struct lm_freq_t {
@@ -229,8 +245,9 @@ PG_HD lm_freq_t lm_freqs(const float* z) {
   const float s = f_add(f_add(e[0], e[1]), e[2]);
   lm_freq_t t;
   for (int c = 0; c < 3; c++) {
-    const float q = f_mul(f_div(e[c], s), float(kLmProbTotal - 3));
-    t.f[c] = 1 + (q >= 1.f ? uint32_t(q) : 0u);
+    // (0 / s apart: a division takes its slow way for a numerator of 0)
+    const float q = f_mul(f_div(e[c] > 0.f ? e[c] : 1.f, s), float(kLmProbTotal - 3));
+    t.f[c] = 1 + (q >= 1.f && e[c] > 0.f ? lm_trunc(q) : 0u);
   }
   int big = 0;
   if (t.f[1] > t.f[big]) big = 1;
