@@ -5,10 +5,9 @@
 // bijection of [0, n) shuffles it; shard s of a power-of-two count holds the
 // shuffled indices congruent to s, at position index >> log2(count).
 //
-// On the GPU: scatter_block for whole batches of blocks (one thread per 32
-// rotations of a node; symbols are written as bytes, one per entry, ready for
-// the format-2 coder), the permutation in both directions, and the board of
-// a shuffled index.
+// On the GPU: scatter_block for whole batches of blocks (symbols are written as
+// bytes, one per entry, ready for the format-2 coder), the permutation in both
+// directions, and the board of a shuffled index.
 #include "../../include/pentago_b200.h"
 #include "lines.h"
 #include "runtime.h"
@@ -41,6 +40,7 @@ struct perm_t {
   uint64_t n, pow2k, offset, mask;
   int k;
   int s[8];
+  uint64_t inv[4];   // (1 + 2^b)^-1 mod 2^64 of each pair's second step
 };
 
 PG_HD uint64_t perm_forward(const perm_t& P, uint64_t x) {
@@ -56,22 +56,22 @@ PG_HD uint64_t perm_forward(const perm_t& P, uint64_t x) {
   return x;
 }
 
-// Inverse: (1 + 2^b)^-1 = (1 - 2^b)(1 + 2^2b)(1 + 2^4b)... mod 2^k, and
+// Inverse, in 32-bit arithmetic (U) where n allows: the second step of a pair
+// is a product, undone by another; the first has
 // (I + R^a)^-1 = (I + R^a)(I + R^2a)(I + R^4a)... over GF(2).
-PG_HD uint64_t perm_inverse(const perm_t& P, uint64_t x) {
+template<class U> PG_HD U perm_inverse_in(const perm_t& P, U x) {
 #pragma unroll
   for (int pair = 3; pair >= 0; pair--) {
     const bool high = pair & 1;
-    if (high ? x < P.offset : x >= P.pow2k) continue;
-    uint64_t t = high ? x - P.offset : x;
-    const int a = P.s[2 * pair], b = P.s[2 * pair + 1];
-    t = (t - (t << b)) & P.mask;
-    for (int c = 2 * b; c < P.k; c *= 2) t = (t + (t << c)) & P.mask;
-    for (int c = a; c < P.k; c *= 2) t ^= t >> c;
-    x = high ? t + P.offset : t;
+    const U offset = high ? U(P.offset) : U(0);
+    const bool inside = high ? x >= offset : x <= U(P.mask);
+    U t = U((x - offset) * U(P.inv[pair])) & U(P.mask);
+    for (int c = P.s[2 * pair]; c < P.k; c *= 2) t ^= t >> c;
+    x = inside ? U(t + offset) : x;
   }
   return x;
 }
+PG_HD uint64_t perm_inverse(const perm_t& P, uint64_t x) { return perm_inverse_in<uint64_t>(P, x); }
 
 // Sections of a slice in the mapping's order (all_boards_sections(slice, 8),
 // pentago/base/all_boards.cc:160-203: standardized sections sorted by
@@ -121,6 +121,11 @@ const slice_map& slice_mapping(int slice) {
   P.mask = P.pow2k - 1;
   P.offset = P.n - P.pow2k;
   for (int i = 0; i < 8; i++) P.s[i] = kPermShifts[slice][i];
+  for (int i = 0; i < 4; i++) {   // (1 + v)^-1 = (1 - v)(1 + v^2)(1 + v^4)...
+    uint64_t v = uint64_t(1) << P.s[2 * i + 1], m = 1 - v;
+    for (v *= v; v; v *= v) m *= 1 + v;
+    P.inv[i] = m;
+  }
   return cache.emplace(slice, std::move(M)).first->second;
 }
 
@@ -206,37 +211,42 @@ PG_HD int64_t shard_start(const int64_t* shard_off, uint64_t n, int shift, int l
   return (s - lo) * q + (std::min<int64_t>(s, r) - std::min<int64_t>(lo, r));
 }
 
-// scatter_block (shard.cc:405-464) for a batch of blocks: thread t of grid
-// row b handles node t >> 3 of block b, rotations 32 (t & 7) .. + 31.
+// The node of a block that thread t of its grid row handles (node t >> 3,
+// rotations 32 (t & 7) .. + 31): its position in its section's row-major order.
+PG_HD uint64_t node_position(const shard_dev_t& D, const block_dev_t& B, int64_t node) {
+  uint64_t pos = 0, scale = 1;
+  for (int q = 3; q >= 0; q--) {
+    pos += scale * uint64_t(B.base[q] + int(node % B.shape[q]));
+    node /= B.shape[q];
+    scale *= uint64_t(ldg(D.shape + 4 * B.section + q));
+  }
+  return pos;
+}
+PG_HD void node_wins(const uint32_t* p, int w, int turn, uint32_t& black, uint32_t& white) {
+  const uint32_t a = p[w], c = p[8 + w];
+  if (turn == 0) { black = a; white = ~c; }
+  else if (turn == 1) { black = ~c; white = a; }
+  else { black = a; white = c; }
+}
+
+// scatter_block (shard.cc:405-464) for a batch of blocks that is part of a
+// slice, entry by entry.  Bound by the single bytes it writes: the L2 takes
+// about 50 G/s of them, wherever they lie.
 __global__ void __launch_bounds__(256)
 shard_scatter_kernel(const shard_dev_t D, const block_dev_t* __restrict__ blocks, int block0,
                      const uint32_t* __restrict__ nodes, int turn, int shift, int lo, int hi,
                      const int64_t* __restrict__ shard_off, uint8_t* __restrict__ symbols) {
   const block_dev_t B = blocks[block0 + blockIdx.y];
   const int64_t nodes_in_block = int64_t(B.shape[0]) * B.shape[1] * B.shape[2] * B.shape[3];
-  const int sshape[4] = {ldg(D.shape + 4 * B.section), ldg(D.shape + 4 * B.section + 1),
-                         ldg(D.shape + 4 * B.section + 2), ldg(D.shape + 4 * B.section + 3)};
   const uint64_t sec_off = ldg(D.offsets + B.section);
   const uint64_t smask = (uint64_t(1) << shift) - 1;
   for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < 8 * nodes_in_block;
        t += int64_t(gridDim.x) * blockDim.x) {
     const int64_t node = t >> 3;
     const int w = int(t & 7);
-    // position of the node: row-major over the section's shape
-    int64_t r = node;
-    int idx[4];
-    for (int q = 3; q >= 0; q--) {
-      idx[q] = B.base[q] + int(r % B.shape[q]);
-      r /= B.shape[q];
-    }
-    const uint64_t pos = ((uint64_t(idx[0]) * sshape[1] + idx[1]) * sshape[2] + idx[2]) * sshape[3] + idx[3];
-    const uint32_t* p = nodes + 16 * (B.node_offset + node);
-    const uint32_t a = p[w], c = p[8 + w];
     uint32_t black, white;
-    if (turn == 0) { black = a; white = ~c; }
-    else if (turn == 1) { black = ~c; white = a; }
-    else { black = a; white = c; }
-    const uint64_t base = sec_off + 256 * pos + 32 * w;
+    node_wins(nodes + 16 * (B.node_offset + node), w, turn, black, white);
+    const uint64_t base = sec_off + 256 * node_position(D, B, node) + 32 * w;
     for (int bit = 0; bit < 32; bit++) {
       const uint64_t y = perm_forward(D.perm, base + bit);
       const int s = int(y & smask);
@@ -244,6 +254,84 @@ shard_scatter_kernel(const shard_dev_t D, const block_dev_t* __restrict__ blocks
       symbols[shard_start(shard_off, D.perm.n, shift, lo, s) + int64_t(y >> shift)] =
           uint8_t((black >> bit & 1) + 2 * (white >> bit & 1));
     }
+  }
+}
+
+// A batch that is a whole slice is taken the other way round: its entries
+// are laid out by linear index first, 2 bits each (black, white), and the
+// shards then written in order, each byte looked up by the inverse
+// permutation.
+PG_HD uint64_t spread16(uint32_t v) {   // bit i of the low 16 to bit 2 i
+  v = (v | v << 8) & 0x00ff00ffu;
+  v = (v | v << 4) & 0x0f0f0f0fu;
+  v = (v | v << 2) & 0x33333333u;
+  return (v | v << 1) & 0x55555555u;
+}
+__global__ void __launch_bounds__(256)
+shard_linear_kernel(const shard_dev_t D, const block_dev_t* __restrict__ blocks, int block0,
+                    const uint32_t* __restrict__ nodes, int turn, uint2* __restrict__ linear) {
+  const block_dev_t B = blocks[block0 + blockIdx.y];
+  const int64_t nodes_in_block = int64_t(B.shape[0]) * B.shape[1] * B.shape[2] * B.shape[3];
+  const uint64_t sec_off = ldg(D.offsets + B.section);
+  for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < 8 * nodes_in_block;
+       t += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t node = t >> 3;
+    const int w = int(t & 7);
+    uint32_t black, white;
+    node_wins(nodes + 16 * (B.node_offset + node), w, turn, black, white);
+    linear[sec_off / 32 + 8 * node_position(D, B, node) + w] =
+        make_uint2(uint32_t(spread16(black & 0xffff) | spread16(white & 0xffff) << 1),
+                   uint32_t(spread16(black >> 16) | spread16(white >> 16) << 1));
+  }
+}
+
+// Entries of shards lo .. hi - 1 in order, 256 a warp and turn (8 a thread, so
+// that 8 lookups are in flight).  Bound by the lookups, sectors of 32 bytes at
+// random places of n / 4 bytes.  Slice 9 into 1,024
+// shards (3.55 G entries, 0.9 GB of them): 59 G lookups/s, 72 ms by bytes, 60 ms now; slice 7
+// (in L2): 180 G/s, 3.6 ms before, 0.8 now; one shard of slice 9: 12.9 ms
+// before, 2.8 now.
+constexpr int kGather = 8;
+template<class U> __global__ void __launch_bounds__(256)
+shard_gather_kernel(const perm_t P, const uint32_t* __restrict__ linear, int shift, int lo, int hi, int64_t total,
+                    const int64_t* __restrict__ shard_off, uint8_t* __restrict__ symbols) {
+  const int lane = threadIdx.x & 31;
+  const int64_t q = int64_t(P.n >> shift), r = int64_t(P.n & ((uint64_t(1) << shift) - 1));
+  const int64_t warps = int64_t(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t span = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); span * 32 * kGather < total;
+       span += warps) {
+    // shard and place in it of the thread's first entry: shards below r have q + 1 entries, the rest q
+    const int64_t first = span * 32 * kGather + lane, longer = std::max<int64_t>(0, std::min<int64_t>(r, hi) - lo) * (q + 1);
+    int64_t s, pos;
+    if (first < longer) {
+      s = lo + U(first) / U(q + 1);
+      pos = U(first) % U(q + 1);
+    } else {
+      const int64_t past = first - longer;
+      s = std::max<int64_t>(r, lo) + (q ? int64_t(U(past) / U(q)) : hi);
+      pos = q ? U(past) % U(q) : 0;
+    }
+    uint32_t word[kGather];
+    int sub[kGather];
+    int64_t to[kGather];
+#pragma unroll
+    for (int i = 0; i < kGather; i++) {
+      while (s < hi && pos >= q + (s < r)) {
+        pos -= q + (s < r);
+        s++;
+      }
+      to[i] = -1;
+      if (s < hi) {
+        to[i] = shard_start(shard_off, P.n, shift, lo, int(s)) + pos;
+        const U x = perm_inverse_in<U>(P, U(uint64_t(pos) << shift | uint64_t(s)));
+        word[i] = ldg(linear + (x >> 4));
+        sub[i] = int(x & 15);
+      }
+      pos += 32;
+    }
+#pragma unroll
+    for (int i = 0; i < kGather; i++)
+      if (to[i] >= 0) symbols[to[i]] = uint8_t(word[i] >> (2 * sub[i]) & 3);
   }
 }
 
@@ -271,6 +359,35 @@ int upload_slice(const slice_map& M, stream_scratch& scratch, cudaStream_t strea
   D.shape = sh;
   D.rmin = rm;
   return PG_OK;
+}
+
+// A batch of blocks of one size that holds every node of the slice once.
+bool whole_slice(const slice_map& M, const pg_shard_block_t* blocks, const std::vector<block_dev_t>& bd) {
+  const int bs = blocks[0].block_size;
+  uint64_t nodes = 0;
+  for (size_t i = 0; i < bd.size(); i++) {
+    if (blocks[i].block_size != bs) return false;
+    nodes += uint64_t(bd[i].shape[0]) * bd[i].shape[1] * bd[i].shape[2] * bd[i].shape[3];
+  }
+  if (256 * nodes != M.perm.n) return false;
+  std::vector<int64_t> first(M.sigs.size() + 1, 0);   // of each section's blocks, and how many along its axes
+  std::vector<int> grid(4 * M.sigs.size());
+  for (size_t i = 0; i < M.sigs.size(); i++) {
+    int sh[4];
+    section_t::from_sig(M.sigs[i]).shape(sh);
+    int64_t k = 1;
+    for (int q = 0; q < 4; q++) k *= grid[4 * i + q] = (sh[q] + bs - 1) / bs;
+    first[i + 1] = first[i] + k;
+  }
+  std::vector<bool> seen(first.back());
+  for (size_t i = 0; i < bd.size(); i++) {
+    int64_t at = 0;
+    for (int q = 0; q < 4; q++) at = at * grid[4 * bd[i].section + q] + blocks[i].block[q];
+    at += first[bd[i].section];
+    if (seen[at]) return false;
+    seen[at] = true;
+  }
+  return true;
 }
 
 bool slice_ok(int slice) { return 0 <= slice && slice <= 18; }
@@ -373,11 +490,30 @@ extern "C" int pg_shard_scatter(int slice, int total_shards, int shard_lo, int s
   }
   const int shift = __builtin_ctz(unsigned(total_shards));
   const int64_t threads = 8 * max_nodes;
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(nodes);
+  uint2* linear = nullptr;
+  if (whole_slice(M, blocks, bd) && scratch.alloc(&linear, M.perm.n / 4) != cudaSuccess) {
+    (void)cudaGetLastError();   // no room for it: entry by entry
+    linear = nullptr;
+  }
   for (int b0 = 0; b0 < nblocks; b0 += 65535) {
     const int nb = std::min(65535, nblocks - b0);
     const unsigned gx = unsigned(std::max<int64_t>(1, std::min<int64_t>((threads + 255) / 256, std::max(1, 148 * 16 / nb))));
-    shard_scatter_kernel<<<dim3(gx, unsigned(nb)), 256, 0, stream>>>(D, bdev, b0, reinterpret_cast<const uint32_t*>(nodes),
-                                                                    turn, shift, shard_lo, shard_hi, off, symbols);
+    const dim3 grid(gx, unsigned(nb));
+    if (linear) shard_linear_kernel<<<grid, 256, 0, stream>>>(D, bdev, b0, words, turn, linear);
+    else shard_scatter_kernel<<<grid, 256, 0, stream>>>(D, bdev, b0, words, turn, shift, shard_lo, shard_hi, off, symbols);
+    PG_CUDA(cudaGetLastError());
+  }
+  if (linear) {
+    int64_t total = 0;
+    const int64_t n = int64_t(M.perm.n), per = n >> shift, more = n & (total_shards - 1);
+    total = (shard_hi - shard_lo) * per + std::min<int64_t>(shard_hi, more) - std::min<int64_t>(shard_lo, more);
+    const unsigned grid = grid_for((total + kGather - 1) / kGather);
+    const uint32_t* at = reinterpret_cast<const uint32_t*>(linear);
+    if (M.perm.n <= 0xffffffffu)
+      shard_gather_kernel<uint32_t><<<grid, 256, 0, stream>>>(M.perm, at, shift, shard_lo, shard_hi, total, off, symbols);
+    else
+      shard_gather_kernel<uint64_t><<<grid, 256, 0, stream>>>(M.perm, at, shift, shard_lo, shard_hi, total, off, symbols);
     PG_CUDA(cudaGetLastError());
   }
   return PG_OK;
