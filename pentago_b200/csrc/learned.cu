@@ -159,42 +159,49 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 // ---------------------------------------------------------------------------
 // Coding: logits on the tensor cores (tcgen05, tensor memory)
 
-// Tables of a coding CTA, from a base of 1,024 bytes.  The B operands are
-// K-major rows of 64 bf16 in the 128-byte swizzle (chunk c of row j at
+// Tables and operands of a coding CTA, from a base of 1,024 bytes.  The
+// operands of the products are K-major rows of 64 bf16 in the 128-byte swizzle (chunk c of row j at
 // c ^ (j & 7)): w1t row k holds W1[72 ..][k] / 16, w2t row i holds W2[..][j] of
-// the unit j that accumulator column i is, lm_unit(i).
+// the unit j that accumulator column i is, lm_unit(i); operand[t] the 128
+// rows of tile t.
 struct lm_coder {
   uint4 w1t[kLmHidden][8];
   uint4 w2t[kLmHidden][8];
-  uint2 near[256];            // per symbol: its 8 neighbours, a byte each
+  uint4 operand[2][128][8];
   float b1[kLmHidden];
-  uint64_t mbar;
+  uint64_t mbar[2];
   uint32_t tmem;
-  int32_t stream[2];
-  uint32_t other[2][32];      // what the second warp of a pair hands to the first
+  uint32_t pad[3];
 };
 
 // Accumulator columns are ordered so that columns 2 i and 2 i + 1 belong to the
 // chains P_t and P_t+1 (t even) of layer 3: one packed operation serves both.
 __host__ __device__ __forceinline__ int lm_unit(int column) { return (column & ~7) + 2 * (column & 3) + (column >> 2 & 1); }
 
-// Layer 3 and the biases beside it, per pair of accumulator columns: a kernel
-// parameter, so that they are operands in constant memory (read from shared
-// memory, each by 32 lanes at once, they took as long as the arithmetic).
-struct lm_out_t {
-  struct { float b2[2], w3[3][2]; } at[kLmHidden / 2];
+// What all threads read at the same place, as a kernel parameter (read from
+// shared memory, by 32 lanes at once, layer 3's weights took as long as its
+// arithmetic): layer 3 and the biases beside it, per pair of accumulator
+// columns, and where each step finds its symbols' neighbours.
+struct lm_const {
+  struct alignas(16) { float b2[2], w3[3][2]; } at[kLmHidden / 2];
+  uint32_t near[128][4];   // per neighbour of symbol st 16 bits: its word in the row | lm_symbol16's rotation << 8
   float b3[4];
 };
-static lm_out_t lm_out(const uint8_t* model) {
+static lm_const lm_consts(const uint8_t* model) {
   auto w = [&](int i) {
     const uint8_t* p = model + kLmModelHeader + 2 * i;
     return bf16_value(uint16_t(p[0] | p[1] << 8));
   };
-  lm_out_t O = {};
+  lm_const O = {};
   for (int i = 0; i < kLmHidden; i++) {
     O.at[i >> 1].b2[i & 1] = w(kLmB2 + lm_unit(i));
     for (int c = 0; c < 3; c++) O.at[i >> 1].w3[c][i & 1] = w(kLmW3 + lm_unit(i) * kLmOut + c);
   }
+  for (int st = 0; st < 128; st++)
+    for (int n = 0; n < 8; n++) {
+      const int a = lm_neighbour(st, n);
+      O.near[st][n >> 1] |= uint32_t((a >> 4) | ((2 * a - 4) & 31) << 8) << (16 * (n & 1));
+    }
   for (int c = 0; c < 3; c++) O.b3[c] = w(kLmB3 + c);
   return O;
 }
@@ -217,76 +224,69 @@ __device__ void lm_build_coder(lm_coder& S, const uint16_t* __restrict__ P, int 
     S.w1t[j][swz(j, c)] = make_uint4(u[0], u[1], u[2], u[3]);
     S.w2t[j][swz(j, c)] = make_uint4(v[0], v[1], v[2], v[3]);
   }
-  for (int r = tid; r < 256; r += nt) {
-    uint32_t at[2] = {0, 0};
-    for (int n = 0; n < 8; n++) at[n >> 2] |= uint32_t(lm_neighbour(r, n)) << (8 * (n & 3));
-    S.near[r] = make_uint2(at[0], at[1]);
-  }
   for (int i = tid; i < kLmHidden; i += nt) S.b1[i] = w(kLmB1 + i);
   // (read by the tensor cores)
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
-// Tensor memory of a CTA, by column: the accumulators of its 128 rows, then
-// the A operand (two bf16 to a column); a warp reads and writes its 32 lanes.
-constexpr uint32_t kLmTmemCols = 128, kLmAcc = 0, kLmOperand = 64;
+// Tensor memory of a CTA, by column: the accumulators of its two tiles of 128
+// rows; a warp reads its 32 lanes.
+constexpr uint32_t kLmTmemCols = 128;
 // Instruction descriptor: fp32 accumulators, bf16 A and B, both K-major, N = 64, M = 128.
 constexpr uint32_t kLmIdesc = 1u << 4 | 1u << 7 | 1u << 10 | (kLmHidden / 8) << 17 | (128 / 16) << 24;
 
-// Shared-memory descriptor of a table: 128-byte swizzle, groups of 8 rows 1,024 bytes apart.
-__device__ __forceinline__ uint64_t lm_desc(const void* table) {
-  const uint64_t a = __cvta_generic_to_shared(table);
+// Shared-memory descriptor of an operand: 128-byte swizzle, groups of 8 rows 1,024 bytes apart.
+__device__ __forceinline__ uint64_t lm_desc(const void* rows) {
+  const uint64_t a = __cvta_generic_to_shared(rows);
   return (a >> 4) | uint64_t(1) << 16 | uint64_t(1024 >> 4) << 32 | uint64_t(1) << 46 | uint64_t(2) << 61;
 }
-// accumulators = operand x table (K = 64, in steps of 16), then an arrival on the barrier; one thread.
+// Tile t's accumulators = operand x table (K = 64, in steps of 16), then an
+// arrival on its barrier: one thread of warp t (a product takes its thread
+// some 300 cycles to issue).
 __device__ __forceinline__ void lm_product(lm_coder& S, const void* table) {
+  const int t = int(threadIdx.x >> 5);
+  if (t >= 2 || (threadIdx.x & 31)) return;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint64_t desc = lm_desc(table);
+  const uint64_t a = lm_desc(S.operand[t]), b = lm_desc(table);
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %4, 0;\n"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-                 :: "r"(S.tmem + kLmAcc), "r"(S.tmem + kLmOperand + 8 * k), "l"(desc + 2 * k), "r"(kLmIdesc),
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                 :: "r"(S.tmem + kLmHidden * t), "l"(a + 2 * k), "l"(b + 2 * k), "r"(kLmIdesc),
                     "r"(uint32_t(k > 0)) : "memory");
   }
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-               :: "r"(unsigned(__cvta_generic_to_shared(&S.mbar))) : "memory");
+               :: "r"(unsigned(__cvta_generic_to_shared(&S.mbar[t]))) : "memory");
 }
-// Waits for a product; false if it has not come after a bounded number of polls.
-__device__ __forceinline__ bool lm_product_wait(lm_coder& S, uint32_t& phase) {
-  const unsigned bar = unsigned(__cvta_generic_to_shared(&S.mbar));
+// Waits for a tile's product; false if it has not come after a bounded number of polls.
+__device__ __forceinline__ bool lm_product_wait(lm_coder& S, int t, uint32_t phase) {
+  const unsigned bar = unsigned(__cvta_generic_to_shared(&S.mbar[t]));
   uint32_t done = 0;
   for (int poll = 0; poll < (1 << 20) && !done; poll++)
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.b32 %0, 1, 0, p;\n}\n"
                  : "=r"(done) : "r"(bar), "r"(phase) : "memory");
-  phase ^= 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   return done != 0;
 }
 
-#define PG_R8(v, b) "r"(v[b]), "r"(v[b + 1]), "r"(v[b + 2]), "r"(v[b + 3]), "r"(v[b + 4]), "r"(v[b + 5]), "r"(v[b + 6]), "r"(v[b + 7])
 #define PG_W8(v, b) "=r"(v[b]), "=r"(v[b + 1]), "=r"(v[b + 2]), "=r"(v[b + 3]), "=r"(v[b + 4]), "=r"(v[b + 5]), "=r"(v[b + 6]), "=r"(v[b + 7])
-// 32 columns of the thread's row (the wait belongs to the load: nothing may use the registers before it).
-__device__ __forceinline__ void tmem_ld(uint32_t* v, uint32_t at) {
+// 32 columns of the thread's row, or 16 each of two places (the wait belongs to
+// the load: nothing may use the registers before it).
+__device__ __forceinline__ void tmem_ld32(uint32_t* v, uint32_t at) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
                "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
                "tcgen05.wait::ld.sync.aligned;\n"
                : PG_W8(v, 0), PG_W8(v, 8), PG_W8(v, 16), PG_W8(v, 24) : "r"(at) : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t at, const uint32_t* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-               "%14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};\n"
-               :: "r"(at), PG_R8(v, 0), PG_R8(v, 8), PG_R8(v, 16), PG_R8(v, 24) : "memory");
+__device__ __forceinline__ void tmem_ld16x2(uint32_t* v, uint32_t* w, uint32_t at, uint32_t bt) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+               "%14, %15}, [%32];\n"
+               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
+               "%28, %29, %30, %31}, [%33];\n"
+               "tcgen05.wait::ld.sync.aligned;\n"
+               : PG_W8(v, 0), PG_W8(v, 8), PG_W8(w, 0), PG_W8(w, 8) : "r"(at), "r"(bt) : "memory");
 }
-__device__ __forceinline__ void tmem_st8(uint32_t at, const uint32_t* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n"
-               :: "r"(at), PG_R8(v, 0) : "memory");
-}
-#undef PG_R8
 #undef PG_W8
-__device__ __forceinline__ void tmem_stored() {
-  asm volatile("tcgen05.wait::st.sync.aligned;\ntcgen05.fence::before_thread_sync;\n" ::: "memory");
-}
 
 // Two fp32 operations, each rounded as usual, in one instruction.
 __device__ __forceinline__ uint64_t f2(float a, float b) { return uint64_t(f_raw(b)) << 32 | f_raw(a); }
@@ -332,65 +332,247 @@ __device__ __forceinline__ uint32_t lm_act_q2(float a, float s, float b, float t
   return d;
 }
 
-// Frequencies of symbol r of the thread's node, given the symbols coded
-// before it: row has 16 v per symbol, 48 for those not coded yet (like a value of
-// 3), prev the previous node's; node: the node's sums / 16.  The CTA's 128
-// threads are the 128 rows of the products and come here together.  Returns
-// false for all of them if a product did not come.
-constexpr int kLmChunk = 32;   // accumulator columns read at a time
-__device__ __forceinline__ bool lm_step_freqs(lm_coder& S, const lm_out_t& O, const uint8_t* row, const uint8_t* prev,
-                                              int r, const float* node, uint32_t& phase, bool& ok, lm_freq_t& F) {
-  const uint32_t tm = S.tmem + (threadIdx.x >> 5 << 21);   // the warp's lanes
-  {
-    uint32_t op[32];
-#pragma unroll
-    for (int q = 0; q < 4; q++) onehot4(op + 2 * q, uint32_t(r >> (2 * q) & 3) << 4);
-    const uint2 at = S.near[r];
-#pragma unroll
-    for (int n = 0; n < 8; n++) onehot4(op + 8 + 2 * n, row[(n < 4 ? at.x : at.y) >> (8 * (n & 3)) & 255]);
-    onehot4(op + 24, prev[r]);
-#pragma unroll
-    for (int i = 26; i < 32; i++) op[i] = 0;
-    tmem_st32(tm + kLmOperand, op);
+// The coding kernels give a stream a warp: lane l has the node of the stream's
+// lane l, whose two symbols of a step (neither is the other's neighbour) are
+// row m of the CTA's two tiles, 128 rows of four streams.  All warps of a CTA
+// take their steps together; nodes have 128 steps, so the streams of a CTA
+// begin their nodes together, and a warp without a stream keeps step
+// without coding.
+//
+// Dynamic shared memory: the tables and operands, then per warp two buffers
+// of its nodes' symbols (the nodes being coded and the ones before them; 2
+// bits a symbol, 3: not coded yet, 17 words a lane so that lanes reading the
+// same rotation use different banks) and, for the decoder, a window of the
+// stream's next words.
+//
+// Bound by the instructions of a step, 1,700 a warp, and their chain: 7,500
+// cycles for three warps a scheduler, of which the operands take 900, the
+// products 700 each, activations 900, layer 3 1,300, the frequencies 1,000 and the
+// states 700.  2,048 blocks of a solved slice: 166 ms each way with mma.sync
+// (256 products a step and stream), 87 with two warps per stream, one tile
+// and the operands in tensor memory (6 streams an SM instead of 12), 75 now.
+constexpr int kLmCodeThreads = 128;
+constexpr int kLmRowWords = 17;
+constexpr int kLmWordWin = 512;   // the decoder's window of upcoming stream words
+constexpr size_t kLmStreamSmem = size_t(2) * 32 * 4 * kLmRowWords + 2 * kLmWordWin;
+constexpr size_t kLmCodeSmem = 1024 + sizeof(lm_coder) + 4 * kLmStreamSmem;   // (from a multiple of 1,024)
+constexpr int kLmCodeCtas = 3;
+static_assert(sizeof(lm_coder) % 16 == 0 && kLmStreamSmem % 16 == 0, "coding rows stay aligned");
+static_assert(kLmCodeCtas * kLmTmemCols <= 512, "tensor memory of an SM");
+
+struct lm_warp {   // a thread's place, and its warp's buffers
+  int lane;
+  uint32_t* row[2];
+  uint16_t* win;
+  __device__ __forceinline__ void fill(uint32_t* to) const {
+    for (int w = 0; w < 16; w++) to[w] = 0xffffffffu;
   }
-  tmem_stored();
-  if (__syncthreads_or(!ok)) return false;
-  if (threadIdx.x == 0) lm_product(S, S.w1t);
-  ok &= lm_product_wait(S, phase);
+  // A node's 256 symbols between global memory and its row; true if one is above 2.
+  __device__ __forceinline__ bool in(uint32_t* to, const uint8_t* g) const {
+    bool bad = false;
+    const bool aligned = (reinterpret_cast<uintptr_t>(g) & 3) == 0;
+#pragma unroll 2
+    for (int w = 0; w < 16; w++) {
+      uint32_t word = 0;
 #pragma unroll
-  for (int h = 0; h < kLmHidden; h += kLmChunk) {
-    uint32_t acc[kLmChunk], op[kLmChunk / 2];
-    tmem_ld(acc, tm + kLmAcc + h);
-#pragma unroll
-    for (int i = 0; i < kLmChunk / 2; i++)
-      op[i] = lm_act_q2(node[h + 2 * i], f_bits(acc[2 * i]), node[h + 2 * i + 1], f_bits(acc[2 * i + 1]));
-#pragma unroll
-    for (int i = 0; i < kLmChunk / 2; i += 8) tmem_st8(tm + kLmOperand + h / 2 + i, op + i);
+      for (int k = 0; k < 4; k++) {
+        const uint8_t* from = g + 16 * w + 4 * k;
+        const uint32_t v = aligned ? *reinterpret_cast<const uint32_t*>(from)
+                                   : from[0] | from[1] << 8 | from[2] << 16 | uint32_t(from[3]) << 24;
+        bad |= (v & 0xfcfcfcfcu) != 0 || (v & v >> 1 & 0x01010101u) != 0;   // a byte above 2
+        word |= ((v & 3) | (v >> 6 & 0xc) | (v >> 12 & 0x30) | (v >> 18 & 0xc0)) << (8 * k);
+      }
+      to[w] = word;
+    }
+    return bad;
   }
-  tmem_stored();
+  __device__ __forceinline__ void out(const uint32_t* from, uint8_t* g) const {
+    const bool aligned = (reinterpret_cast<uintptr_t>(g) & 3) == 0;
+#pragma unroll 2
+    for (int w = 0; w < 16; w++) {
+      const uint32_t word = from[w];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const uint32_t b = word >> (8 * k), v = (b & 3) | (b & 0xc) << 6 | (b & 0x30) << 12 | (b & 0xc0) << 18;
+        uint8_t* at = g + 16 * w + 4 * k;
+        if (aligned) *reinterpret_cast<uint32_t*>(at) = v;
+        else
+          for (int e = 0; e < 4; e++) at[e] = uint8_t(v >> (8 * e));
+      }
+    }
+  }
+};
+
+// The next stream of a launch, largest first (streams are handed to warps one
+// at a time through a counter, in the order the host sorted them), or -1.
+__device__ __forceinline__ int lm_next_stream(int* next, const int32_t* order, int nstreams, int lane) {
+  int k = 0;
+  if (lane == 0) k = atomicAdd(next, 1);
+  k = __shfl_sync(0xffffffffu, k, 0);
+  return k < nstreams ? order[k] : -1;
+}
+
+__device__ __forceinline__ uint32_t lm_symbol16(uint32_t word, uint32_t rotation) {   // 16 v, given v's word
+  return __funnelshift_r(word, word, rotation) & 48u;
+}
+
+// lm_freqs of two rows' logits at once, operation by operation.
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t f2_both(float v) { return f2(v, v); }
+__device__ __forceinline__ void lm_freqs2(const uint64_t* z, lm_freq_t* F) {
+  auto top = [](float a, float b, float c) {   // (a NaN is passed over unless it comes first)
+    a = b > a ? b : a;
+    return c > a ? c : a;
+  };
+  const uint64_t m = f2(top(f2_lo(z[0]), f2_lo(z[1]), f2_lo(z[2])), top(f2_hi(z[0]), f2_hi(z[1]), f2_hi(z[2])));
+  uint64_t e[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {   // lm_exp2
+    const uint64_t d = f2_mul(f2_fma(m, f2_both(-1.f), z[c]), f2_both(1.44269504f));
+    uint64_t u;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(u) : "l"(d), "l"(f2_both(12582912.f)));
+    const uint64_t t = f2_fma(f2_add(u, f2_both(-12582912.f)), f2_both(-1.f), d);
+    uint64_t p = f2_both(1.5252734e-05f);
+    p = f2_fma(p, t, f2_both(1.5403530e-04f));
+    p = f2_fma(p, t, f2_both(1.3333558e-03f));
+    p = f2_fma(p, t, f2_both(9.6181291e-03f));
+    p = f2_fma(p, t, f2_both(5.5504109e-02f));
+    p = f2_fma(p, t, f2_both(2.4022651e-01f));
+    p = f2_fma(p, t, f2_both(6.9314718e-01f));
+    p = f2_fma(p, t, f2_both(1.0f));
+    p = f2_mul(p, f2(f_bits((uint32_t(u) << 23) + 0x3f800000u), f_bits((uint32_t(u >> 32) << 23) + 0x3f800000u)));
+    e[c] = f2(f2_lo(d) >= -24.f ? f2_lo(p) : 0.f, f2_hi(d) >= -24.f ? f2_hi(p) : 0.f);
+  }
+  const uint64_t s = f2_add(f2_add(e[0], e[1]), e[2]);
+#pragma unroll
+  for (int row = 0; row < 2; row++) {
+    auto half = [&](uint64_t v) { return row ? f2_hi(v) : f2_lo(v); };
+    uint32_t f[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float a = half(e[c]), q = f_mul(f_div(a > 0.f ? a : 1.f, half(s)), float(kLmProbTotal - 3));
+      f[c] = 1 + (a > 0.f ? lm_trunc(q) : 0u);
+    }
+    const uint32_t rest = kLmProbTotal - (f[0] + f[1] + f[2]);
+    const bool one = f[1] > f[0], two = f[2] > (one ? f[1] : f[0]);
+    f[0] += one || two ? 0 : rest;
+    f[1] += one && !two ? rest : 0;
+    f[2] += two ? rest : 0;
+    F[row].f[0] = f[0];
+    F[row].f[1] = f[1];
+    F[row].f[2] = f[2];
+    F[row].cum[0] = 0;
+    F[row].cum[1] = f[0];
+    F[row].cum[2] = f[0] + f[1];
+  }
+}
+
+// Row m of both tiles' operands for step st: the one-hot features of symbols st
+// and st + 128 (rotation, neighbours, the previous node's symbol, zeros), a
+// chunk of two features after the other.
+__device__ __forceinline__ void lm_operands(lm_coder& S, const lm_const& O, const uint32_t* row, const uint32_t* prev, int st, int m) {
+  // (all loads before the first store, which the compiler may not move them past)
+  uint32_t sym[2][10];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    // (a symbol 128 on is 8 words on, in the same place)
+    const uint32_t near = O.near[st][c], a = near & 15, b = near >> 16 & 15;
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+      sym[t][2 * c] = lm_symbol16(row[a ^ 8 * t], near >> 8);
+      sym[t][2 * c + 1] = lm_symbol16(row[b ^ 8 * t], near >> 24);
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    sym[t][8] = lm_symbol16(prev[(st >> 4) + 8 * t], 2 * st - 4);
+    sym[t][9] = 64;   // (none)
+  }
+#pragma unroll
+  for (int t = 0; t < 2; t++) {
+    auto put = [&](int c, uint32_t a16, uint32_t b16) {
+      uint32_t op[4];
+      onehot4(op, a16);
+      onehot4(op + 2, b16);
+      S.operand[t][m][swz(m, c)] = make_uint4(op[0], op[1], op[2], op[3]);
+    };
+    const int r = st + 128 * t;
+    put(0, uint32_t(r & 3) << 4, uint32_t(r >> 2 & 3) << 4);
+    put(1, uint32_t(r >> 4 & 3) << 4, uint32_t(r >> 6 & 3) << 4);
+#pragma unroll
+    for (int c = 0; c < 5; c++) put(2 + c, sym[t][2 * c], sym[t][2 * c + 1]);
+    S.operand[t][m][swz(m, 7)] = make_uint4(0, 0, 0, 0);
+  }
+}
+
+// Frequencies of the two symbols of step st of the thread's node.  row has the
+// node's symbols, prev the previous node's; node: the node's sums / 16.  The
+// CTA's 128 threads are the rows of the products and come here together.
+// Returns false for all of them if a product did not come.
+__device__ __forceinline__ bool lm_step_freqs(lm_coder& S, const lm_const& O, const uint32_t* row, const uint32_t* prev,
+                                              int st, const float* node, uint32_t& phase, bool& ok, lm_freq_t* F) {
+  const int m = threadIdx.x;
+  const uint32_t tm = S.tmem + (uint32_t(m) >> 5 << 21);   // the warp's lanes
+  lm_operands(S, O, row, prev, st, m);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (__syncthreads_or(!ok)) return false;
-  if (threadIdx.x == 0) lm_product(S, S.w2t);
-  ok &= lm_product_wait(S, phase);
-  uint64_t part[2][3] = {};   // P_0 and P_1, P_2 and P_3
+  lm_product(S, S.w1t);
 #pragma unroll
-  for (int h = 0; h < kLmHidden; h += kLmChunk) {
-    uint32_t acc[kLmChunk];
-    tmem_ld(acc, tm + kLmAcc + h);
+  for (int t = 0; t < 2; t++) {
+    ok &= lm_product_wait(S, t, phase);
 #pragma unroll
-    for (int i = 0; i < kLmChunk / 2; i++) {
+    for (int h = 0; h < kLmHidden; h += 32) {
+      uint32_t acc[32], op[16];
+      tmem_ld32(acc, tm + kLmHidden * t + h);
+#pragma unroll
+      for (int i = 0; i < 16; i++)
+        op[i] = lm_act_q2(node[h + 2 * i], f_bits(acc[2 * i]), node[h + 2 * i + 1], f_bits(acc[2 * i + 1]));
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        S.operand[t][m][swz(m, h / 8 + c)] = make_uint4(op[4 * c], op[4 * c + 1], op[4 * c + 2], op[4 * c + 3]);
+    }
+  }
+  phase ^= 1;
+  asm volatile("tcgen05.fence::before_thread_sync;\nfence.proxy.async.shared::cta;" ::: "memory");
+  if (__syncthreads_or(!ok)) return false;
+  lm_product(S, S.w2t);
+  ok &= lm_product_wait(S, 0, phase);
+  ok &= lm_product_wait(S, 1, phase);
+  phase ^= 1;
+  // Layer 3 of both rows at once, each constant used twice: P_0 and P_1, P_2 and P_3
+  uint64_t part[2][2][3] = {};
+#pragma unroll
+  for (int h = 0; h < kLmHidden; h += 16) {
+    uint32_t acc[2][16];
+    tmem_ld16x2(acc[0], acc[1], tm + h, tm + kLmHidden + h);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
       const auto& o = O.at[h / 2 + i];
-      const uint64_t a = f2_fma(uint64_t(acc[2 * i + 1]) << 32 | acc[2 * i], f2(kLmActInv, kLmActInv), f2(o.b2[0], o.b2[1]));
-      const uint64_t v = f2(relu(f2_lo(a)), relu(f2_hi(a)));
 #pragma unroll
-      for (int c = 0; c < 3; c++) part[i & 1][c] = f2_fma(f2(o.w3[c][0], o.w3[c][1]), v, part[i & 1][c]);
+      for (int t = 0; t < 2; t++) {
+        const uint64_t a =
+            f2_fma(uint64_t(acc[t][2 * i + 1]) << 32 | acc[t][2 * i], f2(kLmActInv, kLmActInv), f2(o.b2[0], o.b2[1]));
+        const uint64_t v = f2(relu(f2_lo(a)), relu(f2_hi(a)));
+#pragma unroll
+        for (int c = 0; c < 3; c++) part[t][i & 1][c] = f2_fma(f2(o.w3[c][0], o.w3[c][1]), v, part[t][i & 1][c]);
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  float z[3];
+  uint64_t z[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++)
-    z[c] = f_add(O.b3[c], f_add(f_add(f2_lo(part[0][c]), f2_hi(part[0][c])), f_add(f2_lo(part[1][c]), f2_hi(part[1][c]))));
-  F = lm_freqs(z);
+  for (int c = 0; c < 3; c++) {
+    auto chains = [&](int i) {   // of both rows, each the sum of its two
+      const uint64_t a = part[0][i][c], b = part[1][i][c];
+      return f2_add(f2(f2_lo(a), f2_lo(b)), f2(f2_hi(a), f2_hi(b)));
+    };
+    z[c] = f2_add(f2(O.b3[c], O.b3[c]), f2_add(chains(0), chains(1)));
+  }
+  lm_freqs2(z, F);
   return true;
 }
 
@@ -425,106 +607,23 @@ __device__ __forceinline__ uint32_t get32(const uint8_t* p) {
   return uint32_t(p[0]) | uint32_t(p[1]) << 8 | uint32_t(p[2]) << 16 | uint32_t(p[3]) << 24;
 }
 
-// The coding kernels give a stream two warps, which code the two symbols of a
-// step side by side (neither is the other's neighbour): lane l of both has
-// the node of the stream's lane l, the second warp hands its frequencies to
-// the first, and that one keeps the rANS states.  A CTA is two such pairs,
-// 128 rows for one product of the tensor cores.  All its warps take their
-// steps together; nodes have 128 steps, so the streams of a CTA begin
-// their nodes together, and a pair without a stream keeps step without
-// coding.
-//
-// Dynamic shared memory: the tables, then per pair two buffers of its nodes'
-// symbols (the nodes being coded and the ones before them; a row of 256 bytes
-// a lane, rows 260 bytes apart so that lanes reading the same rotation use
-// different banks) and, for the decoder, a window of the stream's next words.
-//
-// Bound by the chain of a step: 5,000 cycles with three CTAs an SM, of which
-// the products take 500 each (issue to arrival), layer 3 900, the frequencies 770, the states 900; its
-// instructions alone would take about 2,000.  2,048 blocks of a solved slice:
-// 166 ms each way with mma.sync (whose 256 products a step and stream were
-// most of it), 87 ms now.  Four CTAs of 128 registers: 100 ms.
-constexpr int kLmSymRow = 260;
-constexpr int kLmWordWin = 1024;   // the decoder's window of upcoming stream words
-constexpr size_t kLmPairSmem = size_t(2) * 32 * kLmSymRow + 2 * kLmWordWin;
-constexpr size_t kLmCodeSmem = 1024 + sizeof(lm_coder) + 2 * kLmPairSmem;   // (from a multiple of 1,024)
-constexpr int kLmCodeCtas = 3;
-static_assert(sizeof(lm_coder) % 16 == 0 && kLmPairSmem % 16 == 0, "coding rows stay aligned");
-static_assert(kLmCodeCtas * kLmTmemCols <= 512, "tensor memory of an SM");
-
-struct lm_pair {   // a thread's place, and its pair's buffers
-  int pair, half, lane;
-  uint8_t* row[2];
-  uint16_t* win;
-  // (a barrier named by a register would reserve all 16 of the CTA's, and with them the SM's room for other CTAs)
-  __device__ __forceinline__ void sync() const {
-    if (pair) asm volatile("bar.sync 2, 64;" ::: "memory");
-    else asm volatile("bar.sync 1, 64;" ::: "memory");
-  }
-  // The pair's threads share a row's words, or its bytes
-  __device__ __forceinline__ void fill(uint8_t* to) const {
-    for (int w = half; w < 64; w += 2) reinterpret_cast<uint32_t*>(to)[w] = 0x30303030u;
-  }
-  // A node's 256 symbols between global memory and its row (16 v there); true if one is above 2.
-  __device__ __forceinline__ bool in(uint8_t* to, const uint8_t* g) const {
-    bool bad = false;
-    if ((reinterpret_cast<uintptr_t>(g) & 3) == 0) {
-#pragma unroll 8
-      for (int w = half; w < 64; w += 2) {
-        const uint32_t v = reinterpret_cast<const uint32_t*>(g)[w];
-        bad |= (v & 0xfcfcfcfcu) != 0 || (v & v >> 1 & 0x01010101u) != 0;   // a byte above 2
-        reinterpret_cast<uint32_t*>(to)[w] = (v & 0x03030303u) << 4;
-      }
-    } else {
-      for (int k = half; k < 256; k += 2) {
-        const uint8_t v = g[k];
-        bad |= v > 2;
-        to[k] = uint8_t((v & 3) << 4);
-      }
-    }
-    return bad;
-  }
-  __device__ __forceinline__ void out(const uint8_t* from, uint8_t* g) const {
-    if ((reinterpret_cast<uintptr_t>(g) & 3) == 0) {
-#pragma unroll 8
-      for (int w = half; w < 64; w += 2)
-        reinterpret_cast<uint32_t*>(g)[w] = reinterpret_cast<const uint32_t*>(from)[w] >> 4 & 0x03030303u;
-    } else {
-      for (int k = half; k < 256; k += 2) g[k] = uint8_t(from[k] >> 4);
-    }
-  }
-  // The next stream of a launch, largest first (streams are handed out one at
-  // a time through a counter, in the order the host sorted them), or -1.
-  __device__ __forceinline__ int next_stream(lm_coder& S, int* next, const int32_t* order, int nstreams) const {
-    if (half == 0 && lane == 0) {
-      const int k = atomicAdd(next, 1);
-      S.stream[pair] = k < nstreams ? order[k] : -1;
-    }
-    sync();
-    const int s = S.stream[pair];
-    sync();
-    return s;
-  }
-};
-
-// Tables, tensor memory and barrier of a coding CTA; and giving them back.
-__device__ lm_coder& lm_coder_begin(unsigned char* raw, const uint16_t* __restrict__ P, lm_pair& W) {
+// Tables, tensor memory and barriers of a coding CTA; and giving them back.
+__device__ lm_coder& lm_coder_begin(unsigned char* raw, const uint16_t* __restrict__ P, lm_warp& W) {
   unsigned char* base = raw + ((1024 - (__cvta_generic_to_shared(raw) & 1023)) & 1023);
   lm_coder& S = *reinterpret_cast<lm_coder*>(base);
   const int warp = threadIdx.x >> 5;
-  W.pair = warp >> 1;
-  W.half = warp & 1;
   W.lane = threadIdx.x & 31;
-  unsigned char* mine = base + sizeof(lm_coder) + kLmPairSmem * W.pair;
-  for (int b = 0; b < 2; b++) W.row[b] = mine + (32 * b + W.lane) * kLmSymRow;
-  W.win = reinterpret_cast<uint16_t*>(mine + 2 * 32 * kLmSymRow);
+  unsigned char* mine = base + sizeof(lm_coder) + kLmStreamSmem * warp;
+  for (int b = 0; b < 2; b++) W.row[b] = reinterpret_cast<uint32_t*>(mine) + (32 * b + W.lane) * kLmRowWords;
+  W.win = reinterpret_cast<uint16_t*>(mine + 2 * 32 * 4 * kLmRowWords);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                  :: "r"(unsigned(__cvta_generic_to_shared(&S.tmem))), "r"(kLmTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(unsigned(__cvta_generic_to_shared(&S.mbar))) : "memory");
+    for (int t = 0; t < 2; t++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(unsigned(__cvta_generic_to_shared(&S.mbar[t]))) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   lm_build_coder(S, P, threadIdx.x, blockDim.x);
@@ -551,17 +650,25 @@ __device__ __forceinline__ void lm_coder_node(const lm_coder& S, const uint16_t*
   for (int k = 0; k < kLmHidden; k++) node[k] = f_mul(node[k], kLmActInv);
 }
 
-// Append one 16-bit word per renormalizing lane, in lane order (encoder).
-__device__ __forceinline__ void lm_put_state(uint32_t& x, uint32_t f, uint32_t cum, bool active, uint8_t* words,
-                                             uint32_t& len, unsigned below) {
+// Append one 16-bit word per renormalizing lane, in lane order, as long as
+// there is room (encoder); inv is 1 / f, rounded.
+__device__ __forceinline__ void lm_put_state(uint32_t& x, uint32_t f, float inv, uint32_t cum, bool active, uint8_t* words,
+                                             uint32_t room, uint32_t& len, unsigned below) {
   const bool emit = active && x >= (f << 17);
   const unsigned mask = __ballot_sync(0xffffffffu, emit);
   if (emit) {
-    put16(words + 2 * (len + __popc(mask & below)), uint16_t(x));
+    const uint32_t at = len + __popc(mask & below);
+    if (at < room) put16(words + 2 * size_t(at), uint16_t(x));
     x >>= 16;
   }
   len += __popc(mask);
-  if (active) x = ((x / f) << kLmProbBits) + x % f + cum;
+  // x / f < 2^17: an estimate by the reciprocal is off by less than 2^-4, so
+  // its integer part by one at most
+  uint32_t q = __float2uint_rz(f_mul(__uint2float_rz(x), inv));
+  int r = int(x - q * f);
+  q += r < 0 ? ~0u : r >= int(f) ? 1u : 0u;
+  r += r < 0 ? int(f) : r >= int(f) ? -int(f) : 0;
+  if (active) x = (q << kLmProbBits) + uint32_t(r) + cum;
 }
 
 // Decode one symbol per active lane and take this step's words (decoder);
@@ -591,14 +698,15 @@ __device__ __forceinline__ int lm_get_symbol(uint32_t& x, uint32_t f0, uint32_t 
 
 // sizes[s] = stream bytes, or PG_ERR_ARG for a symbol above 2 or a symbol
 // count that does not match.
-__global__ void __launch_bounds__(kLmThreads, kLmCodeCtas)
+__global__ void __launch_bounds__(kLmCodeThreads, kLmCodeCtas)
 lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t* __restrict__ blocks, int nstreams,
                  const int32_t* __restrict__ order, int* __restrict__ next, const uint8_t* __restrict__ symbols,
                  const int64_t* __restrict__ offsets, uint8_t* __restrict__ out,
-                 const int64_t* __restrict__ out_offsets, int64_t* __restrict__ sizes, const dev_tables_t T,
-                 const __grid_constant__ lm_out_t O) {
+                 const int64_t* __restrict__ out_offsets, const int64_t* __restrict__ caps,
+                 const int64_t* __restrict__ alt_sizes, int64_t* __restrict__ sizes, const dev_tables_t T,
+                 const __grid_constant__ lm_const O) {
   extern __shared__ __align__(16) unsigned char lm_smem_raw[];
-  lm_pair W;
+  lm_warp W;
   lm_coder& S = lm_coder_begin(lm_smem_raw, P, W);
   const unsigned below = (1u << W.lane) - 1;
   int s = -1, cur = 0;
@@ -607,40 +715,38 @@ lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
   int64_t n = 0, R = 0, round = -1;   // R: the run of nodes of each lane
   const uint8_t* sym0 = nullptr;
   uint8_t *base = nullptr, *words = nullptr;
-  uint32_t x = kLmLower, len = 0;
+  uint32_t x = kLmLower, len = 0, room = 0;
   int bad = 0;
   lm_block_t B = {};
   while (whole) {
     while (more && round < 0) {
       if (s >= 0) {   // the stream is done
-        if (W.half) S.other[W.pair][W.lane] = uint32_t(bad);
-        W.sync();
-        if (!W.half) {
-          put32(base + 20 + 4 * W.lane, x);
-          bad = __any_sync(0xffffffffu, bad | int(S.other[W.pair][W.lane]));
-          if (W.lane == 0) {
-            put32(base, kLmVersion);
-            put32(base + 4, uint32_t(hash));
-            put32(base + 8, uint32_t(hash >> 32));
-            put32(base + 12, uint32_t(n));
-            put32(base + 16, len);
-            sizes[s] = bad ? PG_ERR_ARG : kLmStreamHeader + 2 * int64_t(len);
-          }
+        put32(base + 20 + 4 * W.lane, x);
+        bad = __any_sync(0xffffffffu, bad);
+        if (W.lane == 0) {
+          put32(base, kLmVersion);
+          put32(base + 4, uint32_t(hash));
+          put32(base + 8, uint32_t(hash >> 32));
+          put32(base + 12, uint32_t(n));
+          put32(base + 16, len);
+          sizes[s] = bad ? PG_ERR_ARG : kLmStreamHeader + 2 * int64_t(len);
         }
       }
-      s = W.next_stream(S, next, order, nstreams);
+      s = lm_next_stream(next, order, nstreams, W.lane);
       more = s >= 0;
       if (!more) break;
       B = blocks[s];
       n = B.nodes;
       if (offsets[s + 1] - offsets[s] != 256 * n) {
-        if (W.half == 0 && W.lane == 0) sizes[s] = PG_ERR_ARG;
+        if (W.lane == 0) sizes[s] = PG_ERR_ARG;
         s = -1;
         continue;
       }
       sym0 = symbols + offsets[s];
       base = out + out_offsets[s];
       words = base + kLmStreamHeader;
+      const int64_t end = caps[s] - (alt_sizes[s] > 0 ? alt_sizes[s] : 0) - kLmStreamHeader;   // (bytes)
+      room = end > 0 ? uint32_t(end / 2) : 0u;
       x = kLmLower;
       len = 0;
       bad = 0;
@@ -654,51 +760,52 @@ lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
     const bool active = more && i < n;
     float node[kLmHidden];
     lm_coder_node(S, P, B, i, active, T, node);
-    uint8_t* row = W.row[cur];
-    const uint8_t* prev = W.row[cur ^ 1];
+    uint32_t* row = W.row[cur];
+    const uint32_t* prev = W.row[cur ^ 1];
     if (more) {
       if (round == 0) W.fill(W.row[cur ^ 1]);
       else if (i - 1 < n) bad |= W.in(W.row[cur ^ 1], sym0 + 256 * (i - 1));
-      W.sync();
     }
     for (int st = 127; st >= 0; st--) {
-      const int r = st + 128 * W.half;
-      lm_freq_t F;
-      whole = lm_step_freqs(S, O, row, prev, r, node, phase, ok, F);
+      lm_freq_t F[2];
+      whole = lm_step_freqs(S, O, row, prev, st, node, phase, ok, F);
       if (!whole) break;
-      const int v = row[r] >> 4;
-      row[r] = 48;   // to the earlier steps' symbols, one that is not coded yet
-      uint32_t f = v == 1 ? F.f[1] : v == 2 ? F.f[2] : F.f[0], cum = v == 1 ? F.cum[1] : v == 2 ? F.cum[2] : 0u;
-      if (W.half) S.other[W.pair][W.lane] = f | cum << 16;
-      W.sync();
-      if (!W.half) {
-        // the decoder takes s then s + 128, so the encoder puts s + 128 first
-        const uint32_t o = S.other[W.pair][W.lane];
-        lm_put_state(x, o & 0xffff, o >> 16, active, words, len, below);
-        lm_put_state(x, f, cum, active, words, len, below);
+      // the decoder takes s then s + 128, so the encoder puts s + 128 first
+      uint32_t f[2], cum[2];
+      float inv[2];
+#pragma unroll
+      for (int t = 0; t < 2; t++) {
+        uint32_t& word = row[(st >> 4) + 8 * t];
+        const int v = int(word >> (2 * (st & 15)) & 3);
+        word |= 3u << (2 * (st & 15));   // to the earlier steps' symbols, one that is not coded yet
+        f[t] = v == 1 ? F[t].f[1] : v == 2 ? F[t].f[2] : F[t].f[0];
+        cum[t] = v == 1 ? F[t].cum[1] : v == 2 ? F[t].cum[2] : 0u;
+        inv[t] = __frcp_rn(float(f[t]));
       }
+      lm_put_state(x, f[1], inv[1], cum[1], active, words, room, len, below);
+      lm_put_state(x, f[0], inv[0], cum[0], active, words, room, len, below);
     }
     cur ^= 1;
     round--;
   }
-  if (!whole && s >= 0 && W.half == 0 && W.lane == 0) sizes[s] = PG_ERR_CUDA;
+  if (!whole && s >= 0 && W.lane == 0) sizes[s] = PG_ERR_CUDA;
   lm_coder_end(S);
 }
 
 // status[s] = symbols decoded, or PG_ERR_FORMAT / PG_ERR_CAPACITY.  Version-2
 // streams are left to the format-2 decoder (and streams too short to carry a
 // version, which it rejects).
-__global__ void __launch_bounds__(kLmThreads, kLmCodeCtas)
+__global__ void __launch_bounds__(kLmCodeThreads, kLmCodeCtas)
 lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t* __restrict__ blocks, int nstreams,
                  const int32_t* __restrict__ order, int* __restrict__ next, const uint8_t* __restrict__ in,
                  const int64_t* __restrict__ in_offsets,
                  const int64_t* __restrict__ in_sizes, uint8_t* __restrict__ symbols,
                  const int64_t* __restrict__ sym_offsets, const int64_t* __restrict__ sym_caps,
-                 int64_t* __restrict__ status, const dev_tables_t T, const __grid_constant__ lm_out_t O) {
+                 int64_t* __restrict__ status, const dev_tables_t T, const __grid_constant__ lm_const O) {
   extern __shared__ __align__(16) unsigned char lm_smem_raw[];
-  lm_pair W;
+  lm_warp W;
   lm_coder& S = lm_coder_begin(lm_smem_raw, P, W);
-  const bool first = W.half == 0 && W.lane == 0;
+  const bool first = W.lane == 0;
   const unsigned above = W.lane == 31 ? 0u : ~0u << (W.lane + 1);
   int s = -1, cur = 0;
   bool more = true, ok = true, whole = true;
@@ -712,14 +819,14 @@ lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
   lm_block_t B = {};
   while (whole) {
     while (more && round == R) {
-      if (s >= 0 && !W.half) {
+      if (s >= 0) {
         // A well-formed stream ends with every word read and every lane back
         // at the encoder's initial state.
         bad |= x != kLmLower;
         bad = __any_sync(0xffffffffu, bad);
-        if (W.lane == 0) status[s] = (bad || ptr != 0) ? PG_ERR_FORMAT : 256 * n;
+        if (first) status[s] = (bad || ptr != 0) ? PG_ERR_FORMAT : 256 * n;
       }
-      s = W.next_stream(S, next, order, nstreams);
+      s = lm_next_stream(next, order, nstreams, W.lane);
       more = s >= 0;
       if (!more) break;
       const int now = s;
@@ -757,29 +864,26 @@ lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
     const bool active = more && i < n;
     float node[kLmHidden];
     lm_coder_node(S, P, B, i, active, T, node);
-    uint8_t* row = W.row[cur];
+    uint32_t* row = W.row[cur];
     W.fill(row);
-    const uint8_t* prev = W.row[cur ^ 1];   // the previous node of the run is the row of the last round
+    const uint32_t* prev = W.row[cur ^ 1];   // the previous node of the run is the row of the last round
     // the round's words are the last unread ones: stage up to kLmWordWin of them
     const int64_t wlo = ptr > kLmWordWin ? ptr - kLmWordWin : 0;
-    if (more && !W.half) {
+    if (more) {
+      __syncwarp();
 #pragma unroll 4
       for (int64_t w = wlo + W.lane; w < ptr; w += 32) W.win[w - wlo] = get16(words + 2 * w);
+      __syncwarp();
     }
-    if (more) W.sync();
     for (int st = 0; st < 128; st++) {
-      const int r = st + 128 * W.half;
-      lm_freq_t F;
-      whole = lm_step_freqs(S, O, row, prev, r, node, phase, ok, F);
+      lm_freq_t F[2];
+      whole = lm_step_freqs(S, O, row, prev, st, node, phase, ok, F);
       if (!whole) break;
-      if (W.half) S.other[W.pair][W.lane] = F.f[0] | F.f[1] << 16;
-      W.sync();
-      if (!W.half) {
-        const uint32_t o = S.other[W.pair][W.lane];
-        row[st] = uint8_t(lm_get_symbol(x, F.f[0], F.f[1], active, words, W.win, wlo, ptr, above, bad) << 4);
-        row[st + 128] = uint8_t(lm_get_symbol(x, o & 0xffff, o >> 16, active, words, W.win, wlo, ptr, above, bad) << 4);
+#pragma unroll
+      for (int t = 0; t < 2; t++) {   // (the row's symbols are 3 until they are coded)
+        const int v = lm_get_symbol(x, F[t].f[0], F[t].f[1], active, words, W.win, wlo, ptr, above, bad);
+        row[(st >> 4) + 8 * t] ^= uint32_t(v ^ 3) << (2 * (st & 15));
       }
-      W.sync();
     }
     if (active && whole) W.out(row, out0 + 256 * i);
     cur ^= 1;
@@ -822,17 +926,35 @@ lm_freqs_kernel(const uint16_t* __restrict__ P, const lm_block_t* __restrict__ b
   }
 }
 
-// Keep the smaller of the learned and format-2 streams.
-__global__ void lm_choose_kernel(int nstreams, uint8_t* __restrict__ out, const int64_t* __restrict__ out_offsets,
-                                 int64_t* __restrict__ sizes, const uint8_t* __restrict__ alt,
-                                 const int64_t* __restrict__ alt_offsets, const int64_t* __restrict__ alt_sizes) {
+// The encoder keeps the smaller of the learned and format-2 streams.  The
+// format-2 stream is coded first, into its slot, and moved to the slot's end;
+// the learned one is coded from the front and drops the words that would reach
+// into it (it is then the larger one).
+__device__ __forceinline__ void lm_move(uint8_t* to, const uint8_t* from, int64_t n) {   // one CTA; may overlap
+  const bool up = to > from;
+  for (int64_t done = 0; done < n; done += blockDim.x) {
+    const int64_t k = up ? n - 1 - done - threadIdx.x : done + threadIdx.x;
+    const bool mine = k >= 0 && k < n;
+    const uint8_t v = mine ? from[k] : 0;
+    __syncthreads();
+    if (mine) to[k] = v;
+    __syncthreads();
+  }
+}
+__global__ void lm_aside_kernel(uint8_t* __restrict__ out, const int64_t* __restrict__ out_offsets,
+                                const int64_t* __restrict__ caps, const int64_t* __restrict__ alt_sizes) {
+  const int64_t b = alt_sizes[blockIdx.x];
+  uint8_t* slot = out + out_offsets[blockIdx.x];
+  if (b > 0) lm_move(slot + caps[blockIdx.x] - b, slot, b);
+}
+__global__ void lm_choose_kernel(uint8_t* __restrict__ out, const int64_t* __restrict__ out_offsets,
+                                 const int64_t* __restrict__ caps, int64_t* __restrict__ sizes,
+                                 const int64_t* __restrict__ alt_sizes) {
   const int s = blockIdx.x;
-  if (s >= nstreams) return;
   const int64_t a = sizes[s], b = alt_sizes[s];
   if (a < 0 || b < 0 || b >= a) return;
-  uint8_t* d = out + out_offsets[s];
-  const uint8_t* src = alt + alt_offsets[s];
-  for (int64_t k = threadIdx.x; k < b; k += blockDim.x) d[k] = src[k];
+  uint8_t* slot = out + out_offsets[s];
+  lm_move(slot, slot + caps[s] - b, b);
   if (threadIdx.x == 0) sizes[s] = b;
 }
 
@@ -1429,7 +1551,7 @@ static int lm_code_grid(int nstreams) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return std::max(1, std::min((nstreams + 1) / 2, kLmCodeCtas * sms));
+  return std::max(1, std::min((nstreams + 3) / 4, kLmCodeCtas * sms));
 }
 
 }  // namespace pg
@@ -1471,30 +1593,25 @@ extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t
   std::vector<lm_block_t> hb;
   if (int rc = lm_prepare(model, blocks, nstreams, st, L, &hb)) return rc;
   if (int rc = lm_smem_opt_in(lm_encode_kernel, kLmCodeSmem)) return rc;
-  lm_encode_kernel<<<lm_code_grid(nstreams), kLmThreads, kLmCodeSmem, st>>>(
-      L.params, L.hash, L.blocks, nstreams, L.order, L.next, symbols, offsets, out, out_offsets, sizes, *T,
-      lm_out(model));
-  PG_CUDA(cudaGetLastError());
-  // Format-2 streams of the same symbols; the smaller one is kept
-  // alt_off[s] = slot of stream s; alt_off[nstreams + s] = its symbol count
-  std::vector<int64_t> alt_off(2 * nstreams);
-  int64_t total = 0;
+  // What every slot has room for, and its stream's symbol count; then the sizes of the format-2 streams
+  std::vector<int64_t> slots(2 * size_t(nstreams));
   for (int s = 0; s < nstreams; s++) {
-    alt_off[s] = total;
-    alt_off[nstreams + s] = 256 * hb[s].nodes;
-    total += (rans_stream_bound(256 * hb[s].nodes) + 15) & ~15;
+    slots[s] = pg_rans_learned_bound(hb[s].nodes);
+    slots[size_t(nstreams) + s] = 256 * hb[s].nodes;
   }
-  // Scratch for the format-2 streams
   stream_scratch X(st);
-  uint8_t* alt = nullptr;
-  int64_t *alt_off_d = nullptr, *alt_sizes = nullptr;
-  PG_CUDA(X.alloc(&alt, std::max<int64_t>(total, 16)));
-  PG_CUDA(X.alloc(&alt_off_d, sizeof(int64_t) * 2 * nstreams));
-  PG_CUDA(X.alloc(&alt_sizes, sizeof(int64_t) * nstreams));
-  PG_CUDA(cudaMemcpyAsync(alt_off_d, alt_off.data(), sizeof(int64_t) * 2 * nstreams, cudaMemcpyHostToDevice, st));
-  if (int rc = launch_rans_encode(symbols, offsets, nstreams, alt, alt_off_d, alt_sizes, alt_off_d + nstreams, st))
-    return rc;
-  lm_choose_kernel<<<nstreams, 256, 0, st>>>(nstreams, out, out_offsets, sizes, alt, alt_off_d, alt_sizes);
+  int64_t* caps = nullptr;
+  PG_CUDA(X.alloc(&caps, sizeof(int64_t) * 3 * nstreams));
+  int64_t* alt_sizes = caps + 2 * size_t(nstreams);
+  PG_CUDA(cudaMemcpyAsync(caps, slots.data(), sizeof(int64_t) * 2 * nstreams, cudaMemcpyHostToDevice, st));
+  if (int rc = launch_rans_encode(symbols, offsets, nstreams, out, out_offsets, alt_sizes, caps + nstreams, st)) return rc;
+  lm_aside_kernel<<<nstreams, 256, 0, st>>>(out, out_offsets, caps, alt_sizes);
+  PG_CUDA(cudaGetLastError());
+  lm_encode_kernel<<<lm_code_grid(nstreams), kLmCodeThreads, kLmCodeSmem, st>>>(
+      L.params, L.hash, L.blocks, nstreams, L.order, L.next, symbols, offsets, out, out_offsets, caps, alt_sizes, sizes, *T,
+      lm_consts(model));
+  PG_CUDA(cudaGetLastError());
+  lm_choose_kernel<<<nstreams, 256, 0, st>>>(out, out_offsets, caps, sizes, alt_sizes);
   PG_CUDA(cudaGetLastError());
   return PG_OK;
 }
@@ -1513,9 +1630,9 @@ extern "C" int pg_rans_learned_decode(const uint8_t* model, const pg_block_ref_t
   if (int rc = launch_rans_decode(in, in_offsets, in_sizes, nstreams, symbols, sym_offsets, sym_caps, status, 1, st))
     return rc;
   if (int rc = lm_smem_opt_in(lm_decode_kernel, kLmCodeSmem)) return rc;
-  lm_decode_kernel<<<lm_code_grid(nstreams), kLmThreads, kLmCodeSmem, st>>>(
+  lm_decode_kernel<<<lm_code_grid(nstreams), kLmCodeThreads, kLmCodeSmem, st>>>(
       L.params, L.hash, L.blocks, nstreams, L.order, L.next, in, in_offsets, in_sizes, symbols, sym_offsets, sym_caps,
-      status, *T, lm_out(model));
+      status, *T, lm_consts(model));
   PG_CUDA(cudaGetLastError());
   return PG_OK;
 }
