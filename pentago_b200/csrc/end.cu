@@ -370,7 +370,7 @@ template<bool REFL> PG_HD void axis_maps(super8& s, int c0, int c1, int c2) {
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const uint32_t t = ((s.w[i] >> 2) ^ s.w[i]) & m;
-        s.w[i] ^= t ^ (t << 2);
+        s.w[i] ^= imad(t, 5, 0);
       }
     }
     // axis 1 (nibbles of a 16-bit half)
@@ -385,16 +385,17 @@ template<bool REFL> PG_HD void axis_maps(super8& s, int c0, int c1, int c2) {
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const uint32_t t = ((s.w[i] >> 8) ^ s.w[i]) & m;
-        s.w[i] ^= t ^ (t << 8);
+        s.w[i] ^= imad(t, 0x101, 0);
       }
     }
   } else {
     const uint32_t m0 = (0xfu >> c0) * 0x11111111u, m1 = (0xffffu >> (4 * c1)) * 0x10001u;
+    const uint32_t l0 = 16u >> c0, l1 = 0x10000u >> (4 * c1);   // shifts to the left
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       uint32_t x = s.w[i];
-      x = ((x >> c0) & m0) | ((x << (4 - c0)) & ~m0);
-      x = ((x >> (4 * c1)) & m1) | ((x << (16 - 4 * c1)) & ~m1);
+      x = ((x >> c0) & m0) | (imad(x, l0, 0) & ~m0);
+      x = ((x >> (4 * c1)) & m1) | (imad(x, l1, 0) & ~m1);
       s.w[i] = x;
     }
   }

@@ -107,18 +107,34 @@ PG_HD void s_store32(uint64_t* p, const super8& s) {
 #endif
 }
 
+// a * b + c, on the device by an integer multiply-add: the kernels on supers
+// are bound by the pipe that does shifts and logic (74% busy), while the one of
+// multiply-adds is idle (18%), so a shift to the left, or one to the left and an
+// OR of disjoint bits, is better a product.
+PG_HD uint32_t imad(uint32_t a, uint32_t b, uint32_t c) {
+#ifdef __CUDA_ARCH__
+  uint32_t d;
+  asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+#else
+  return a * b + c;
+#endif
+}
+
 // rmax(f)(a) = max over the 8 single rotations b of f(a + b)
 // (pentago/base/superscore.h:10-16): the OR of f shifted by +-1 along each axis.
 PG_HD super8 s_rmax(const super8& f) {
   super8 r;
 #pragma unroll
   for (int i = 0; i < 8; i++) {
+    // Axis 0: at a place of a nibble the OR of its neighbours, the two places of
+    // the other parity.  y has in the nibble's bits 0 and 1 the ORs y0 and y1 of
+    // the even and the odd places; wanted is y1 y0 y1 y0 from bit 0 up, 10 y0 + 5 y1 =
+    // 10 y - 15 y1.  Axis 1 is the same for the nibbles of a halfword.
     const uint32_t x = f.w[i];
-    const uint32_t a0 = ((x >> 1) & 0x77777777u) | ((x << 3) & 0x88888888u) |
-                        ((x << 1) & 0xeeeeeeeeu) | ((x >> 3) & 0x11111111u);
-    const uint32_t a1 = ((x >> 4) & 0x0fff0fffu) | ((x << 12) & 0xf000f000u) |
-                        ((x << 4) & 0xfff0fff0u) | ((x >> 12) & 0x000f000fu);
-    r.w[i] = a0 | a1;
+    const uint32_t y = (x | x >> 2) & 0x33333333u, y1 = y >> 1 & 0x11111111u;
+    const uint32_t z = (x | x >> 8) & 0x00ff00ffu, z1 = z >> 4 & 0x000f000fu;
+    r.w[i] = imad(y, 10, imad(y1, uint32_t(-15), 0)) | imad(z, 0x1010, imad(z1, uint32_t(-0xffff), 0));
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) {
@@ -206,7 +222,7 @@ template<int I, int J> PG_HD void s_swap_bits(super8& s) {
     for (int i = 0; i < 8; i++) {
       const uint32_t x = s.w[i];
       const uint32_t t = ((x >> d) ^ x) & m;
-      s.w[i] = x ^ t ^ (t << d);
+      s.w[i] = x ^ imad(t, 1u + (1u << d), 0);   // (t and t << d share no bit)
     }
   } else if constexpr (I < 5) {
     constexpr int wb = J - 5, sh = 1 << I;
@@ -481,10 +497,11 @@ PG_HD half4 h_rmax(const half4& x) {
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const uint32_t v = x.w[i];
+    // (axis 1 as in s_rmax, for the pairs of bits of a byte)
     const uint32_t t = (v | (v >> 1)) & 0x55555555u;
-    const uint32_t a = t | (t << 1);
-    const uint32_t b = ((v >> 2) & 0x3f3f3f3fu) | ((v << 6) & 0xc0c0c0c0u) |
-                       ((v << 2) & 0xfcfcfcfcu) | ((v >> 6) & 0x03030303u);
+    const uint32_t a = imad(t, 3, 0);
+    const uint32_t y = (v | v >> 4) & 0x0f0f0f0fu, y1 = y >> 2 & 0x03030303u;
+    const uint32_t b = imad(y, 68, imad(y1, uint32_t(-255), 0));
     const uint32_t c = funnel_r(v, v, 8) | funnel_r(v, v, 24);
     r.w[i] = a | b | c;
   }
