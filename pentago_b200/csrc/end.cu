@@ -485,10 +485,22 @@ PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uin
 }
 
 // Parent i of a microline (compute.cc:308-356), in the line frame until its
-// store.  h is the first 16 bytes of its record, rec the record.
+// store.  h is the first 16 bytes of its record, rec the record.  On the
+// device the threads of a pair come here together, each with a parent of its
+// own; the second one's is `real` or, past the last, the first one's again.
+//
+// A node is 64 bytes and nodes are far apart on most axes, so a warp's store
+// of one half of 32 nodes goes through the cache's tags a line at a time, and
+// those passes, with the ones of shared memory, are what sweeps are bound by
+// (about 80% of the cycles).  Each pair of threads therefore trades halves and
+// writes its two nodes one after the other, both halves at once: half as many
+// lines per access, and as many for what is read back when accumulating.
+// Lines of axis 0 of a sweep of 59 M parents: 2.42 ms before, 2.09 now.  On
+// axis 3, where the nodes of a line are neighbours, the trade costs more than
+// it saves (2.48 and 2.59 ms), and each thread writes its own node.
 template<int DIM>
 PG_HD void parent_node(const line_dev_t& L, const microline_geom& G, const uint2* tab0, const uint4* qs,
-                       const uint2* pats, const uint4 h, const uint4* rec, int i, unsigned* errors) {
+                       const uint2* pats, const uint4 h, const uint4* rec, int i, bool real, unsigned* errors) {
   const int p0 = L.npat[0], pp = p0 + L.npat[1];
   // Where the result goes.  Node offsets are multiples of 64 bytes, so a
   // 32-byte aligned output base allows one 256-bit access per super.  When
@@ -544,6 +556,31 @@ PG_HD void parent_node(const line_dev_t& L, const microline_geom& G, const uint2
   super8 r1 = s_or(s_andnot(not_loss, immediate), wins0);
   s_line_frame<DIM>(r0);
   s_line_frame<DIM>(r1);
+#ifdef __CUDA_ARCH__
+  if (DIM < 3 && wide) {
+    // The first thread of a pair takes the win halves, the second the others
+    const bool second = threadIdx.x & 1;
+    const unsigned mask = __activemask();
+    super8 a, b;   // of the first thread's node, of the second's
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+      const uint32_t got = __shfl_xor_sync(mask, second ? r0.w[w] : r1.w[w], 1);
+      a.w[w] = second ? got : r0.w[w];
+      b.w[w] = second ? r1.w[w] : got;
+    }
+    uint64_t* const other = reinterpret_cast<uint64_t*>(__shfl_xor_sync(mask, reinterpret_cast<unsigned long long>(out), 1));
+    uint64_t *const pa = (second ? other : out) + 4 * second, *const pb = (second ? out : other) + 4 * second;
+    const bool both = __shfl_xor_sync(mask, int(real), 1) & int(real);
+    if (accumulate) {
+      a = s_or(s_load32(pa), a);
+      if (both) b = s_or(s_load32(pb), b);
+    }
+    s_store32(pa, a);
+    if (both) s_store32(pb, b);
+    return;
+  }
+#endif
+  if (!real) return;
   if (accumulate) {
     r0 = s_or(wide ? s_load32(out) : s_load(out), r0);
     r1 = s_or(wide ? s_load32(out + 4) : s_load(out + 4), r1);
@@ -709,24 +746,28 @@ __device__ __forceinline__ void cta_microlines(const line_dev_t& L, cta_smem<MIC
   }
   // Each thread's first record header is requested before the barrier, the
   // next one while it computes the current parent.
+  // (nt is even: a pair of threads is the parents 2 m and 2 m + 1; past the last, 2 m again)
+  const int total = M * np;
+  auto parent_of = [&](int x) { return x < total ? x : x - 1; };
   uint4 h = make_uint4(0, 0, 0, 0);
-  if (tid < M * np) {
+  if ((tid & ~1) < total) {
     int k, i;
-    split(tid, np, L.split_m[0], k, i);
+    split(parent_of(tid), np, L.split_m[0], k, i);
     h = ldg(recs + 3 * i);
   }
   __syncthreads();
   unsigned errors = 0;
-  for (int x = tid; x < M * np; x += nt) {
+  for (int x = tid; (x & ~1) < total; x += nt) {
     int k, i;
-    split(x, np, L.split_m[0], k, i);
+    split(parent_of(x), np, L.split_m[0], k, i);
     const uint4 a = h;
-    if (x + nt < M * np) {
+    if (((x + nt) & ~1) < total) {
       int kn, in;
-      split(x + nt, np, L.split_m[0], kn, in);
+      split(parent_of(x + nt), np, L.split_m[0], kn, in);
       h = ldg(recs + 3 * in);
     }
-    parent_node<DIM>(L, S.ctx[k].G, S.tab[k], q_smem + 4 * k * nc, pats + 4 * pp * k, a, recs + 3 * i, i, &errors);
+    parent_node<DIM>(L, S.ctx[k].G, S.tab[k], q_smem + 4 * k * nc, pats + 4 * pp * k, a, recs + 3 * i, i, x < total,
+                     &errors);
   }
   if (errors) record_errors(errors);
 }
@@ -791,7 +832,7 @@ template<int DIM, int G> static unsigned host_line(const line_dev_t& L, const de
       }
     for (int i = 0; i < L.nparent; i++) {
       const uint4* rp = reinterpret_cast<const uint4*>(L.recs + i);
-      parent_node<DIM>(L, geom, tab[0], q.data(), pat.data(), rp[0], rp, i, &errors);
+      parent_node<DIM>(L, geom, tab[0], q.data(), pat.data(), rp[0], rp, i, true, &errors);
     }
   }
   return errors;
