@@ -753,7 +753,9 @@ def main():
         if not args.no_cpu_baseline:
             learned["cpu_static_coder"] = cpu_static_coder_rate(*sample, seconds=5.0)
             sweep2["cpu_baseline"] = cpu_sweep_estimate(SWEEP_ROOT, timings, seconds_per_slice=1.5)
-            sweep2["kernel_speedup_vs_cpu_estimate"] = sweep2["cpu_baseline"]["estimated_s"] / (sweep2["kernel_ms"] / 1e3)
+            if sweep2["cpu_baseline"]:   # (none without the reference engine's library)
+                sweep2["kernel_speedup_vs_cpu_estimate"] = (sweep2["cpu_baseline"]["estimated_s"] /
+                                                            (sweep2["kernel_ms"] / 1e3))
 
     if rank == 0 and world == 1 and not args.no_slice_files:
         # The .pentago slice files: filter kernels alone against the HBM
