@@ -417,6 +417,19 @@ template<int DIM, int G> PG_HD void child_map(super8& a, int c) {
   axis_maps<(G >= 4)>(a, c & 3, c >> 2 & 3, c >> 4 & 3);
 }
 
+// The threads of the warp that take turn x of a loop over `count` pairs of
+// adjacent threads (x: the thread's own place; a warp's places follow one
+// another), as the mask of the turn's shuffles.  It is worked out, not asked
+// for: what a turn does differs from thread to thread, and who happens to be
+// active says nothing about a partner that has not come back together yet,
+// while those that a mask names meet.  (64 lines and a sweep slice 291 us and
+// 5.08 ms; 297 and 5.19 with a mask for each pair, 287 and 5.14 with full
+// masks and whole warps kept in the loops.)
+__device__ __forceinline__ unsigned turn_mask(int x, int count) {
+  const int left = 2 * count - (x - int(threadIdx.x & 31));
+  return left >= 32 ? ~0u : (1u << left) - 1;
+}
+
 PG_HD uint32_t select4(const uint4 v, int i) {
   return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w;
 }
@@ -438,7 +451,7 @@ PG_HD uint32_t select4(const uint4 v, int i) {
 // halves 2 (p nc + j) + half.
 template<int DIM, int G>
 PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uint2* tab0, uint2* q2, int j, int nc,
-                      int half, const super8& x, const uint4 csub) {
+                      int half, const super8& x, const uint4 csub, unsigned mask) {
   super8 z = s_rmax(s_not(x));
   const int c = ladd(geom.base_l, int(L.csym[j]) << 6);   // the translation, axes moved to the line frame
   child_map<DIM, G>(z, c);
@@ -451,8 +464,8 @@ PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uin
 #ifdef __CUDA_ARCH__
   // On the device the two threads of a child each evaluate two of W_j's four
   // word pairs (the not-lost half's pairs 2 and 3 reach the win half by
-  // shuffles), so neither idles while the other does the lookups.  Both
-  // threads of a child are always active together.
+  // shuffles), so neither idles while the other does the lookups.  `mask`
+  // names the threads that are here, both of a child among them.
   {
     uint32_t w[4];
 #pragma unroll
@@ -463,7 +476,6 @@ PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uin
       w[2 * kk] = a.x | b.x | d.x | e.x;
       w[2 * kk + 1] = a.y | b.y | d.y | e.y;
     }
-    const unsigned mask = __activemask();
     uint32_t o[4];
 #pragma unroll
     for (int t = 0; t < 4; t++) o[t] = __shfl_xor_sync(mask, w[t], 1);
@@ -487,7 +499,8 @@ PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uin
 // Parent i of a microline (compute.cc:308-356), in the line frame until its
 // store.  h is the first 16 bytes of its record, rec the record.  On the
 // device the threads of a pair come here together, each with a parent of its
-// own; the second one's is `real` or, past the last, the first one's again.
+// own; the second one's is `real` or, past the last, the first one's again;
+// `mask` names the threads that are here.
 //
 // A node is 64 bytes and nodes are far apart on most axes, so a warp's store
 // of one half of 32 nodes goes through the cache's tags a line at a time, and
@@ -500,7 +513,8 @@ PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uin
 // it saves (2.48 and 2.59 ms), and each thread writes its own node.
 template<int DIM>
 PG_HD void parent_node(const line_dev_t& L, const microline_geom& G, const uint2* tab0, const uint4* qs,
-                       const uint2* pats, const uint4 h, const uint4* rec, int i, bool real, unsigned* errors) {
+                       const uint2* pats, const uint4 h, const uint4* rec, int i, bool real, unsigned mask,
+                       unsigned* errors) {
   const int p0 = L.npat[0], pp = p0 + L.npat[1];
   // Where the result goes.  Node offsets are multiples of 64 bytes, so a
   // 32-byte aligned output base allows one 256-bit access per super.  When
@@ -560,7 +574,6 @@ PG_HD void parent_node(const line_dev_t& L, const microline_geom& G, const uint2
   if (DIM < 3 && wide) {
     // The first thread of a pair takes the win halves, the second the others
     const bool second = threadIdx.x & 1;
-    const unsigned mask = __activemask();
     super8 a, b;   // of the first thread's node, of the second's
 #pragma unroll
     for (int w = 0; w < 8; w++) {
@@ -741,7 +754,8 @@ __device__ __forceinline__ void cta_microlines(const line_dev_t& L, cta_smem<MIC
         cx = child_load(C, child_addr(C, S.ctx[kn].G, jn) + 4 * (1 - half));
         cs = ldg(crecs + jn);
       }
-      child_half<DIM, G>(L, S.ctx[k].G, S.tab[k], reinterpret_cast<uint2*>(q_smem + 4 * k * nc), j, nc, half, v, s);
+      child_half<DIM, G>(L, S.ctx[k].G, S.tab[k], reinterpret_cast<uint2*>(q_smem + 4 * k * nc), j, nc, half, v, s,
+                         turn_mask(x, M * nc));
     }
   }
   // Each thread's first record header is requested before the barrier, the
@@ -767,7 +781,7 @@ __device__ __forceinline__ void cta_microlines(const line_dev_t& L, cta_smem<MIC
       h = ldg(recs + 3 * in);
     }
     parent_node<DIM>(L, S.ctx[k].G, S.tab[k], q_smem + 4 * k * nc, pats + 4 * pp * k, a, recs + 3 * i, i, x < total,
-                     &errors);
+                     turn_mask(x, (total + 1) >> 1), &errors);
   }
   if (errors) record_errors(errors);
 }
@@ -828,11 +842,11 @@ template<int DIM, int G> static unsigned host_line(const line_dev_t& L, const de
         const uint64_t* a = child_addr(child_source(L), geom, j);
         for (int half = 0; half < 2; half++)
           child_half<DIM, G>(L, geom, tab[0], reinterpret_cast<uint2*>(q.data()), j, L.nchild, half,
-                             s_load_ldg(a + 4 * (1 - half)), reinterpret_cast<const uint4*>(L.crecs)[j]);
+                             s_load_ldg(a + 4 * (1 - half)), reinterpret_cast<const uint4*>(L.crecs)[j], 0);
       }
     for (int i = 0; i < L.nparent; i++) {
       const uint4* rp = reinterpret_cast<const uint4*>(L.recs + i);
-      parent_node<DIM>(L, geom, tab[0], q.data(), pat.data(), rp[0], rp, i, true, &errors);
+      parent_node<DIM>(L, geom, tab[0], q.data(), pat.data(), rp[0], rp, i, true, 0, &errors);
     }
   }
   return errors;
