@@ -412,7 +412,13 @@ store_encode_kernel(const uint64_t* __restrict__ nodes, const int64_t* __restric
     if (__any_sync(0xffffffffu, off - int(bits >> 3) < 4)) {
       __syncwarp();
       const int64_t nw = 8 * int64_t(n);
-      for (int64_t i = lane; i < nw; i += kLanesS) reinterpret_cast<uint64_t*>(sbase + kHead)[i] = base[i];
+      uint8_t* raw = sbase + kHead;
+      if ((reinterpret_cast<uintptr_t>(raw) & 7) == 0) {
+        for (int64_t i = lane; i < nw; i += kLanesS) reinterpret_cast<uint64_t*>(raw)[i] = base[i];
+      } else {
+        for (int64_t i = lane; i < nw; i += kLanesS)
+          for (int j = 0; j < 8; j++) raw[8 * i + j] = uint8_t(base[i] >> (8 * j));
+      }
       for (int j = lane; j < kHead; j += 32) sbase[j] = j < 4 ? 0xff : 0;
       if (lane == 0) sizes[b] = kHead + 8 * nw;
       continue;
