@@ -1018,14 +1018,27 @@ template<int ROW> __device__ __forceinline__ void frag_bn(uint32_t* b, const uin
 }
 
 // v = term 0 + term 1 + term 2, bf16 each, exactly (8 bits of v's 24 each),
-// for two values packed per word.
+// for two values packed per word.  Of a value that rounds to an infinity the
+// first term is cut instead; of an infinity or NaN it is that, the others 0.
+__device__ __noinline__ uint32_t split_odd(float v) {
+  const uint32_t u = f_raw(v);
+  return (u & 0x7fffffffu) >= 0x7f7f8000u ? u >> 16 | (v == v ? 0u : 0x40u) : uint32_t(bf16_round_number(v));
+}
 __device__ __forceinline__ void split3(float v0, float v1, uint32_t* term) {
+  term[0] = uint32_t(bf16_round_number(v0)) | uint32_t(bf16_round_number(v1)) << 16;
+  float r0 = f_add(v0, -f_bits(term[0] << 16)), r1 = f_add(v1, -f_bits(term[0] & 0xffff0000u)), most;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(most) : "f"(fabsf(v0)), "f"(fabsf(v1)));
+  if (!(most < 3.38e38f)) {
+    term[0] = split_odd(v0) | split_odd(v1) << 16;
+    r0 = f_finite(v0) ? f_add(v0, -f_bits(term[0] << 16)) : 0.f;
+    r1 = f_finite(v1) ? f_add(v1, -f_bits(term[0] & 0xffff0000u)) : 0.f;
+  }
 #pragma unroll
-  for (int s = 0; s < 3; s++) {
-    const uint16_t a = bf16_round(v0), b = bf16_round(v1);
+  for (int s = 1; s < 3; s++) {
+    const uint16_t a = bf16_round_number(r0), b = bf16_round_number(r1);
     term[s] = uint32_t(a) | uint32_t(b) << 16;
-    v0 = f_add(v0, -bf16_value(a));
-    v1 = f_add(v1, -bf16_value(b));
+    r0 = f_add(r0, -bf16_value(a));
+    r1 = f_add(r1, -bf16_value(b));
   }
 }
 
@@ -1033,9 +1046,16 @@ __device__ __forceinline__ void split3(float v0, float v1, uint32_t* term) {
 // neighbour and previous-node rows and W2 on their column grids, as the
 // exported model holds them (lm_grid_params).  Thread (column, quarter) finds
 // its quarter's largest magnitude, then moves its rows onto the column's grid.
-__device__ __forceinline__ void lm_grad_weights(lm_grad_smem& G, const float* __restrict__ params, int tid) {
-  for (int i = tid; i < kLmRot * kLmHidden; i += kGradThreads)
-    G.w1[i / kLmHidden][i % kLmHidden] = bf16_round(params[kLmW1 + i]);
+// Returns (to all threads) whether the stone rows are finite (the others are, on
+// their grids); weights that are not are 0 here, and lm_odd_stones has them.
+__device__ __forceinline__ bool lm_grad_weights(lm_grad_smem& G, const float* __restrict__ params, int tid) {
+  bool finite = true;
+  for (int i = tid; i < kLmRot * kLmHidden; i += kGradThreads) {
+    const uint16_t w = bf16_round(params[kLmW1 + i]);
+    const bool number = f_finite(bf16_value(w));
+    finite &= number;
+    G.w1[i / kLmHidden][i % kLmHidden] = number ? w : uint16_t(0);
+  }
   for (int i = tid; i < (128 - kLmIn) * kLmHidden; i += kGradThreads) G.w1[kLmIn + i / kLmHidden][i % kLmHidden] = 0;
   if (tid < kLmHidden) {
     G.b1[tid] = bf16_of(params, kLmB1 + tid);
@@ -1064,7 +1084,7 @@ __device__ __forceinline__ void lm_grad_weights(lm_grad_smem& G, const float* __
     top[part][col] = ma;
     top[part][kLmHidden + col] = mb;
   }
-  __syncthreads();
+  finite = __syncthreads_and(finite);
   if (part < 4) {
     auto most = [&](int c) { return fmaxf(fmaxf(top[0][c], top[1][c]), fmaxf(top[2][c], top[3][c])); };
     const float ma = most(col), mb = most(kLmHidden + col);
@@ -1075,6 +1095,7 @@ __device__ __forceinline__ void lm_grad_weights(lm_grad_smem& G, const float* __
 #pragma unroll
     for (int i = 0; i < kB; i++) G.w2[kB * part + i][col] = mb > 0.f ? bf16_round(lm_grid_quantize(b[i], eb)) : 0;
   }
+  return finite;
 }
 
 // Units of the products over samples: 16 x 16 pieces of dW1 (rows 0..127, db1
@@ -1114,6 +1135,33 @@ __device__ __forceinline__ void sample_product(float (*acc)[4], const uint16_t (
   }
 }
 
+// A product with the features multiplies all of a column by a sample's 0s and
+// 1s, and 0 times an infinity is NaN, so what is not finite goes around the
+// products: it reaches a sample from its own features, and their rows from it.
+
+// The sums of those stone weights over the samples of the warp's 16 rows, into
+// the place of the gradient terms (not in use yet): [row][hidden].
+__device__ __noinline__ void lm_odd_stones(lm_grad_smem& G, const float* __restrict__ params, int row0, int lane) {
+  float* sums = reinterpret_cast<float*>(&G.d[0][0][0]) + row0 * kLmHidden;
+  for (int i = lane; i < 16 * kLmHidden; i += 32) {
+    const int row = row0 + i / kLmHidden, k = i % kLmHidden;
+    float s = 0.f;
+    for (int f = 0; f < kLmRot; f++) {
+      const float w = bf16_of(params, kLmW1 + f * kLmHidden + k);
+      if (G.x[row][f] && !f_finite(w)) s += w;
+    }
+    sums[i] = s;
+  }
+  __syncwarp();
+}
+// dL/da1 of a sample's hidden unit k to the rows of its features and to the
+// bias, in the CTA's partial sums (whichever order they come in, sums of
+// infinities and NaN are the same).
+__device__ __noinline__ void lm_odd_gradient(const lm_grad_smem& G, float* out, int row, int k, float v) {
+  for (int f = 0; f <= kOnes; f++)
+    if (G.x[row][f]) atomicAdd(out + (f < kOnes ? kLmW1 + f * kLmHidden + k : kLmB1 + k), v);
+}
+
 __global__ void __launch_bounds__(kGradThreads)
 lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ blocks, int nstreams,
                const uint8_t* __restrict__ symbols, const int64_t* __restrict__ offsets,
@@ -1121,7 +1169,7 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
   extern __shared__ __align__(16) unsigned char lm_smem_raw[];
   lm_grad_smem& G = *reinterpret_cast<lm_grad_smem*>(lm_smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  lm_grad_weights(G, params, tid);
+  const bool finite_stones = lm_grad_weights(G, params, tid);
   for (int i = lane; i < kLmOut * kLmHidden; i += 32) (&G.gw3[warp][0][0])[i] = 0.f;
   float g1[kMine1][2][4] = {}, g2[kMine2][2][4] = {};   // this warp's units of dW1 and dW2
   float gb3[3] = {}, gloss = 0.f;                       // this lane's rows
@@ -1130,6 +1178,8 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
     v += __shfl_xor_sync(0xffffffffu, v, 8);
     return v + __shfl_xor_sync(0xffffffffu, v, 16);
   };
+  float* out = partial + int64_t(blockIdx.x) * (kLmParams + 1);
+  bool odd = false;   // out has what is not finite of dW1 and db1
   const int64_t tiles = (n + kTile - 1) / kTile;
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     // Features: thread 2 s sets the stones of sample s, thread 2 s + 1 the rest
@@ -1197,6 +1247,15 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
         add_part(acc[2 * np + 1], part[1]);
       }
     }
+    if (!finite_stones) {
+      lm_odd_stones(G, params, row0, lane);
+      const float* sums = reinterpret_cast<const float*>(&G.d[0][0][0]) + row0 * kLmHidden;
+#pragma unroll
+      for (int nt = 0; nt < 8; nt++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[nt][i] += sums[(g + 8 * (i >> 1)) * kLmHidden + 8 * nt + 2 * t + (i & 1)];
+      __syncthreads();   // (before the terms are written there)
+    }
     // The activations hq / 16, packed as layer 2's A operand
     uint32_t h[4][4];
 #pragma unroll
@@ -1223,8 +1282,10 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
         mma_bf16(acc[2 * np], h[kt], b[0], b[1]);
         mma_bf16(acc[2 * np + 1], h[kt], b[2], b[3]);
       }
-    // Layer 3, the loss and dL/dz of the two rows (every lane of a quad holds both)
+    // Layer 3, the loss and dL/dz of the two rows (every lane of a quad holds
+    // both); nothing of a row that does not count, whatever the weights are
     float z[2][3] = {};
+    const int ys[2] = {G.y[row0 + g], G.y[row0 + g + 8]};
 #pragma unroll
     for (int nt = 0; nt < 8; nt++)
 #pragma unroll
@@ -1233,7 +1294,7 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
         const float4 w3 = *reinterpret_cast<const float4*>(G.w3[j]);
 #pragma unroll
         for (int half = 0; half < 2; half++) {
-          const float a2 = f_add(G.b2[j], acc[nt][2 * half + e]);
+          const float a2 = ys[half] >= 0 ? f_add(G.b2[j], acc[nt][2 * half + e]) : 0.f;
           acc[nt][2 * half + e] = a2;
           const float r = relu(a2);
           z[half][0] = fmaf(w3.x, r, z[half][0]);
@@ -1250,7 +1311,7 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
         z[half][c] += __shfl_xor_sync(0xffffffffu, z[half][c], 2);
         z[half][c] += G.b3[c];
       }
-      const int y = G.y[row0 + g + 8 * half];
+      const int y = ys[half];
       const float m = fmaxf(z[half][0], fmaxf(z[half][1], z[half][2]));
       float e[3], es = 0.f;
 #pragma unroll
@@ -1335,7 +1396,27 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
       if (unit < 16) sample_product(g2[u], G.h, G.d, 16 * (unit >> 2), 16 * (unit & 3), lane);
       else if (unit < kUnits2) sample_product(g2[u], G.x, G.d, 112, 16 * (unit & 3), lane);
     }
-    __syncthreads();
+    float probe = 0.f;   // 0 if they are all finite
+#pragma unroll
+    for (int nt = 0; nt < 8; nt++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) probe = fmaf(acc[nt][i], 0.f, probe);
+    if (__syncthreads_or(probe != 0.f)) {   // (NaN too)
+      if (!odd) {
+        for (int i = tid; i < kLmW2; i += kGradThreads) __stcg(out + i, 0.f);
+        __threadfence();
+        __syncthreads();
+      }
+      odd = true;
+#pragma unroll
+      for (int nt = 0; nt < 8; nt++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          float& d = acc[nt][i];
+          if (!f_finite(d)) lm_odd_gradient(G, out, row0 + g + 8 * (i >> 1), 8 * nt + 2 * t + (i & 1), d);
+          d = f_finite(d) ? d : 0.f;
+        }
+    }
     // dW1 from their features and dL/da1
 #pragma unroll
     for (int nt = 0; nt < 8; nt++)
@@ -1357,7 +1438,6 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
   }
   // Partial sums of this CTA: the units of dW1 and dW2 (with the biases'
   // rows), then the warps' sums, in order.
-  float* out = partial + int64_t(blockIdx.x) * (kLmParams + 1);
   // Rows r0 .. of a unit at columns c0 ..: row `last` to out + bias, those
   // before it to out + base
   auto put = [&](const float (*acc)[4], int base, int r0, int c0, int last, int bias) {
@@ -1367,7 +1447,10 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
       for (int half = 0; half < 2; half++) {
         const int r = r0 + g + 8 * half, c = c0 + 8 * nt + 2 * t;
         float* o = r < last ? out + base + r * kLmHidden + c : out + bias + c;
-        if (r <= last) { o[0] = acc[nt][2 * half]; o[1] = acc[nt][2 * half + 1]; }
+        if (r > last) continue;
+        const bool add = odd && base == kLmW1;
+        o[0] = acc[nt][2 * half] + (add ? __ldcg(o) : 0.f);
+        o[1] = acc[nt][2 * half + 1] + (add ? __ldcg(o + 1) : 0.f);
       }
   };
 #pragma unroll
