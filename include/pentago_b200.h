@@ -323,7 +323,8 @@ int64_t pg_rans_learned_bound(int64_t nodes);
 
 /* Encode stream s: the symbols[offsets[s] .. offsets[s+1]) of block blocks[s]
  * (256 per node) into out + out_offsets[s] (room for pg_rans_learned_bound),
- * sizes[s] = its bytes or PG_ERR_ARG.  `model` and `blocks` are host arrays;
+ * sizes[s] = its bytes, PG_ERR_ARG, or PG_ERR_CUDA for a stream that the kernel
+ * gave up on.  `model` and `blocks` are host arrays;
  * symbols, offsets, out, out_offsets and sizes are device arrays. */
 int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams, const uint8_t* symbols,
                            const int64_t* offsets, uint8_t* out, const int64_t* out_offsets, int64_t* sizes,
@@ -331,7 +332,8 @@ int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, i
 
 /* Decode stream s (either format) into symbols + sym_offsets[s] (room for
  * sym_caps[s]); status[s] = symbols decoded, PG_ERR_FORMAT (malformed, or
- * coded with another model or for another block) or PG_ERR_CAPACITY. */
+ * coded with another model or for another block), PG_ERR_CAPACITY, or
+ * PG_ERR_CUDA as above. */
 int pg_rans_learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams, const uint8_t* in,
                            const int64_t* in_offsets, const int64_t* in_sizes, uint8_t* symbols,
                            const int64_t* sym_offsets, const int64_t* sym_caps, int64_t* status, void* stream);
@@ -536,6 +538,15 @@ int pg_selftest_midsolve_groups_host(const uint64_t* raws, int n, int groups, pg
  * `polls` polls: the wait runs out and *fault_out = 1 (device check of the
  * bounded barrier the multi-CTA midsolve and the server use). */
 int pg_debug_barrier_timeout(unsigned polls, int* fault_out);
+/* pg_rans_learned_encode / _decode with the wait for each stream's last
+ * tensor-core product taken to have run out: every stream that the learned
+ * coder has to do with ends with PG_ERR_CUDA. */
+int pg_debug_learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams, const uint8_t* symbols,
+                            const int64_t* offsets, uint8_t* out, const int64_t* out_offsets, int64_t* sizes,
+                            void* stream);
+int pg_debug_learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams, const uint8_t* in,
+                            const int64_t* in_offsets, const int64_t* in_sizes, uint8_t* symbols,
+                            const int64_t* sym_offsets, const int64_t* sym_caps, int64_t* status, void* stream);
 /* The shard permutation (op 0 forward, 1 inverse) and boards (op 2) of n
  * host indices, with the kernels' own functions. */
 int pg_selftest_shard_host(int op, int slice, const uint64_t* in, int64_t n, uint64_t* out);

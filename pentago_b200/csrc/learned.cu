@@ -512,14 +512,19 @@ __device__ __forceinline__ void lm_operands(lm_coder& S, const lm_const& O, cons
 // Frequencies of the two symbols of step st of the thread's node.  row has the
 // node's symbols, prev the previous node's; node: the node's sums / 16.  The
 // CTA's 128 threads are the rows of the products and come here together.
-// Returns false for all of them if a product did not come.
+// ok: the thread has seen all its products so far; false is returned to all of
+// them if one of them has not (the caller looks at ok after its last step).
+// phase is the parity of the latest products; with `drill` the wait for the
+// second is taken to have run out.
 __device__ __forceinline__ bool lm_step_freqs(lm_coder& S, const lm_const& O, const uint32_t* row, const uint32_t* prev,
-                                              int st, const float* node, uint32_t& phase, bool& ok, lm_freq_t* F) {
+                                              int st, const float* node, uint32_t& phase, bool& ok, lm_freq_t* F,
+                                              bool drill) {
   const int m = threadIdx.x;
   const uint32_t tm = S.tmem + (uint32_t(m) >> 5 << 21);   // the warp's lanes
   lm_operands(S, O, row, prev, st, m);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   if (__syncthreads_or(!ok)) return false;
+  phase ^= 1;
   lm_product(S, S.w1t);
 #pragma unroll
   for (int t = 0; t < 2; t++) {
@@ -536,13 +541,12 @@ __device__ __forceinline__ bool lm_step_freqs(lm_coder& S, const lm_const& O, co
         S.operand[t][m][swz(m, h / 8 + c)] = make_uint4(op[4 * c], op[4 * c + 1], op[4 * c + 2], op[4 * c + 3]);
     }
   }
-  phase ^= 1;
   asm volatile("tcgen05.fence::before_thread_sync;\nfence.proxy.async.shared::cta;" ::: "memory");
   if (__syncthreads_or(!ok)) return false;
-  lm_product(S, S.w2t);
-  ok &= lm_product_wait(S, 0, phase);
-  ok &= lm_product_wait(S, 1, phase);
   phase ^= 1;
+  lm_product(S, S.w2t);
+  ok &= lm_product_wait(S, 0, phase) && !drill;
+  ok &= lm_product_wait(S, 1, phase);
   // Layer 3 of both rows at once, each constant used twice: P_0 and P_1, P_2 and P_3
   uint64_t part[2][2][3] = {};
 #pragma unroll
@@ -632,7 +636,11 @@ __device__ lm_coder& lm_coder_begin(unsigned char* raw, const uint16_t* __restri
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   return S;
 }
-__device__ void lm_coder_end(lm_coder& S) {
+// `whole`: every product has been seen.  Those that have not are given as long
+// again, so that tensor memory is not freed under them.
+__device__ void lm_coder_end(lm_coder& S, bool whole, uint32_t phase) {
+  if (!whole)
+    for (int t = 0; t < 2; t++) lm_product_wait(S, t, phase);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -697,7 +705,11 @@ __device__ __forceinline__ int lm_get_symbol(uint32_t& x, uint32_t f0, uint32_t 
 }
 
 // sizes[s] = stream bytes, or PG_ERR_ARG for a symbol above 2 or a symbol
-// count that does not match.
+// count that does not match; what it was before (PG_ERR_CUDA) if the stream's
+// CTA, or all of them, gave up on a product.
+// kDrill: the wait for a stream's last product is taken to have run out, to see
+// what then becomes of the streams.
+template<bool kDrill>
 __global__ void __launch_bounds__(kLmCodeThreads, kLmCodeCtas)
 lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t* __restrict__ blocks, int nstreams,
                  const int32_t* __restrict__ order, int* __restrict__ next, const uint8_t* __restrict__ symbols,
@@ -711,7 +723,7 @@ lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
   const unsigned below = (1u << W.lane) - 1;
   int s = -1, cur = 0;
   bool more = true, ok = true, whole = true;
-  uint32_t phase = 0;
+  uint32_t phase = 1;
   int64_t n = 0, R = 0, round = -1;   // R: the run of nodes of each lane
   const uint8_t* sym0 = nullptr;
   uint8_t *base = nullptr, *words = nullptr;
@@ -768,7 +780,7 @@ lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
     }
     for (int st = 127; st >= 0; st--) {
       lm_freq_t F[2];
-      whole = lm_step_freqs(S, O, row, prev, st, node, phase, ok, F);
+      whole = lm_step_freqs(S, O, row, prev, st, node, phase, ok, F, kDrill && st == 0 && round == 0);
       if (!whole) break;
       // the decoder takes s then s + 128, so the encoder puts s + 128 first
       uint32_t f[2], cum[2];
@@ -785,16 +797,18 @@ lm_encode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
       lm_put_state(x, f[1], inv[1], cum[1], active, words, room, len, below);
       lm_put_state(x, f[0], inv[0], cum[0], active, words, room, len, below);
     }
+    if (__syncthreads_or(!ok)) whole = false;   // (the last step's products among them)
     cur ^= 1;
     round--;
   }
-  if (!whole && s >= 0 && W.lane == 0) sizes[s] = PG_ERR_CUDA;
-  lm_coder_end(S);
+  lm_coder_end(S, whole, phase);
 }
 
-// status[s] = symbols decoded, or PG_ERR_FORMAT / PG_ERR_CAPACITY.  Version-2
+// status[s] = symbols decoded, or PG_ERR_FORMAT / PG_ERR_CAPACITY; what it was
+// before (PG_ERR_CUDA) as in the encoder, and kDrill likewise.  Version-2
 // streams are left to the format-2 decoder (and streams too short to carry a
 // version, which it rejects).
+template<bool kDrill>
 __global__ void __launch_bounds__(kLmCodeThreads, kLmCodeCtas)
 lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t* __restrict__ blocks, int nstreams,
                  const int32_t* __restrict__ order, int* __restrict__ next, const uint8_t* __restrict__ in,
@@ -809,7 +823,7 @@ lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
   const unsigned above = W.lane == 31 ? 0u : ~0u << (W.lane + 1);
   int s = -1, cur = 0;
   bool more = true, ok = true, whole = true;
-  uint32_t phase = 0;
+  uint32_t phase = 1;
   int64_t n = 0, R = 0, round = 0;   // R: the run of nodes of each lane
   const uint8_t* words = nullptr;
   uint8_t* out0 = nullptr;
@@ -877,7 +891,7 @@ lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
     }
     for (int st = 0; st < 128; st++) {
       lm_freq_t F[2];
-      whole = lm_step_freqs(S, O, row, prev, st, node, phase, ok, F);
+      whole = lm_step_freqs(S, O, row, prev, st, node, phase, ok, F, kDrill && st == 127 && round == R - 1);
       if (!whole) break;
 #pragma unroll
       for (int t = 0; t < 2; t++) {   // (the row's symbols are 3 until they are coded)
@@ -885,12 +899,12 @@ lm_decode_kernel(const uint16_t* __restrict__ P, uint64_t hash, const lm_block_t
         row[(st >> 4) + 8 * t] ^= uint32_t(v ^ 3) << (2 * (st & 15));
       }
     }
+    if (__syncthreads_or(!ok)) whole = false;   // (the last step's products among them)
     if (active && whole) W.out(row, out0 + 256 * i);
     cur ^= 1;
     round++;
   }
-  if (!whole && s >= 0 && first) status[s] = PG_ERR_CUDA;
-  lm_coder_end(S);
+  lm_coder_end(S, whole, phase);
 }
 
 // Frequencies of given samples (for checking the coding path against the CPU).
@@ -942,8 +956,10 @@ __device__ __forceinline__ void lm_move(uint8_t* to, const uint8_t* from, int64_
   }
 }
 __global__ void lm_aside_kernel(uint8_t* __restrict__ out, const int64_t* __restrict__ out_offsets,
-                                const int64_t* __restrict__ caps, const int64_t* __restrict__ alt_sizes) {
+                                const int64_t* __restrict__ caps, const int64_t* __restrict__ alt_sizes,
+                                int64_t* __restrict__ sizes) {
   const int64_t b = alt_sizes[blockIdx.x];
+  if (threadIdx.x == 0) sizes[blockIdx.x] = PG_ERR_CUDA;   // until the learned coder has been there
   uint8_t* slot = out + out_offsets[blockIdx.x];
   if (b > 0) lm_move(slot + caps[blockIdx.x] - b, slot, b);
 }
@@ -1682,9 +1698,10 @@ extern "C" int pg_learned_export(const float* params, uint8_t* model) {
   return PG_OK;
 }
 
-extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
-                                      const uint8_t* symbols, const int64_t* offsets, uint8_t* out,
-                                      const int64_t* out_offsets, int64_t* sizes, void* stream) {
+template<bool kDrill>
+static int learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
+                          const uint8_t* symbols, const int64_t* offsets, uint8_t* out, const int64_t* out_offsets,
+                          int64_t* sizes, void* stream) {
   if (nstreams < 0 || (nstreams && !blocks)) return fail(PG_ERR_ARG, "bad stream list");
   if (!nstreams) return PG_OK;
   const cudaStream_t st = (cudaStream_t)stream;
@@ -1693,7 +1710,7 @@ extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t
   lm_launch L;
   std::vector<lm_block_t> hb;
   if (int rc = lm_prepare(model, blocks, nstreams, st, L, &hb)) return rc;
-  if (int rc = lm_smem_opt_in(lm_encode_kernel, kLmCodeSmem)) return rc;
+  if (int rc = lm_smem_opt_in(lm_encode_kernel<kDrill>, kLmCodeSmem)) return rc;
   // What every slot has room for, and its stream's symbol count; then the sizes of the format-2 streams
   std::vector<int64_t> slots(2 * size_t(nstreams));
   for (int s = 0; s < nstreams; s++) {
@@ -1706,9 +1723,9 @@ extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t
   int64_t* alt_sizes = caps + 2 * size_t(nstreams);
   PG_CUDA(cudaMemcpyAsync(caps, slots.data(), sizeof(int64_t) * 2 * nstreams, cudaMemcpyHostToDevice, st));
   if (int rc = launch_rans_encode(symbols, offsets, nstreams, out, out_offsets, alt_sizes, caps + nstreams, st)) return rc;
-  lm_aside_kernel<<<nstreams, 256, 0, st>>>(out, out_offsets, caps, alt_sizes);
+  lm_aside_kernel<<<nstreams, 256, 0, st>>>(out, out_offsets, caps, alt_sizes, sizes);
   PG_CUDA(cudaGetLastError());
-  lm_encode_kernel<<<lm_code_grid(nstreams), kLmCodeThreads, kLmCodeSmem, st>>>(
+  lm_encode_kernel<kDrill><<<lm_code_grid(nstreams), kLmCodeThreads, kLmCodeSmem, st>>>(
       L.params, L.hash, L.blocks, nstreams, L.order, L.next, symbols, offsets, out, out_offsets, caps, alt_sizes, sizes, *T,
       lm_consts(model));
   PG_CUDA(cudaGetLastError());
@@ -1717,10 +1734,10 @@ extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t
   return PG_OK;
 }
 
-extern "C" int pg_rans_learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
-                                      const uint8_t* in, const int64_t* in_offsets, const int64_t* in_sizes,
-                                      uint8_t* symbols, const int64_t* sym_offsets, const int64_t* sym_caps,
-                                      int64_t* status, void* stream) {
+template<bool kDrill>
+static int learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams, const uint8_t* in,
+                          const int64_t* in_offsets, const int64_t* in_sizes, uint8_t* symbols,
+                          const int64_t* sym_offsets, const int64_t* sym_caps, int64_t* status, void* stream) {
   if (nstreams < 0 || (nstreams && !blocks)) return fail(PG_ERR_ARG, "bad stream list");
   if (!nstreams) return PG_OK;
   const cudaStream_t st = (cudaStream_t)stream;
@@ -1730,12 +1747,42 @@ extern "C" int pg_rans_learned_decode(const uint8_t* model, const pg_block_ref_t
   if (int rc = lm_prepare(model, blocks, nstreams, st, L)) return rc;
   if (int rc = launch_rans_decode(in, in_offsets, in_sizes, nstreams, symbols, sym_offsets, sym_caps, status, 1, st))
     return rc;
-  if (int rc = lm_smem_opt_in(lm_decode_kernel, kLmCodeSmem)) return rc;
-  lm_decode_kernel<<<lm_code_grid(nstreams), kLmCodeThreads, kLmCodeSmem, st>>>(
+  if (int rc = lm_smem_opt_in(lm_decode_kernel<kDrill>, kLmCodeSmem)) return rc;
+  lm_decode_kernel<kDrill><<<lm_code_grid(nstreams), kLmCodeThreads, kLmCodeSmem, st>>>(
       L.params, L.hash, L.blocks, nstreams, L.order, L.next, in, in_offsets, in_sizes, symbols, sym_offsets, sym_caps,
       status, *T, lm_consts(model));
   PG_CUDA(cudaGetLastError());
   return PG_OK;
+}
+
+extern "C" int pg_rans_learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
+                                      const uint8_t* symbols, const int64_t* offsets, uint8_t* out,
+                                      const int64_t* out_offsets, int64_t* sizes, void* stream) {
+  return learned_encode<false>(model, blocks, nstreams, symbols, offsets, out, out_offsets, sizes, stream);
+}
+
+extern "C" int pg_rans_learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
+                                      const uint8_t* in, const int64_t* in_offsets, const int64_t* in_sizes,
+                                      uint8_t* symbols, const int64_t* sym_offsets, const int64_t* sym_caps,
+                                      int64_t* status, void* stream) {
+  return learned_decode<false>(model, blocks, nstreams, in, in_offsets, in_sizes, symbols, sym_offsets, sym_caps, status,
+                               stream);
+}
+
+// The two with the wait for each stream's last product taken to have run out:
+// what a CTA that gives up leaves behind.
+extern "C" int pg_debug_learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
+                                       const uint8_t* symbols, const int64_t* offsets, uint8_t* out,
+                                       const int64_t* out_offsets, int64_t* sizes, void* stream) {
+  return learned_encode<true>(model, blocks, nstreams, symbols, offsets, out, out_offsets, sizes, stream);
+}
+
+extern "C" int pg_debug_learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,
+                                       const uint8_t* in, const int64_t* in_offsets, const int64_t* in_sizes,
+                                       uint8_t* symbols, const int64_t* sym_offsets, const int64_t* sym_caps,
+                                       int64_t* status, void* stream) {
+  return learned_decode<true>(model, blocks, nstreams, in, in_offsets, in_sizes, symbols, sym_offsets, sym_caps, status,
+                              stream);
 }
 
 extern "C" int pg_learned_freqs(const uint8_t* model, const pg_block_ref_t* blocks, int nstreams,

@@ -573,8 +573,10 @@ rans_decode_kernel(const uint8_t* __restrict__ in, const int64_t* __restrict__ i
     const uint8_t* base = in + in_offsets[s];
     const int64_t size = in_sizes[s];
     // Streams of another version are left to the learned decoder when asked
+    // (whose CTAs that give up say nothing: the status stays this one)
     if (only_v2 && size >= 4 && get_u32(base) != 2) {
       live = false;
+      if (lane == 0) status[s] = PG_ERR_CUDA;
     } else {
       // Header checks as arithmetic_deserialize / arithmetic_decode (arithmetic.cc:403-495)
       int64_t bad = 0;
