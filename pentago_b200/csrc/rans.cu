@@ -6,6 +6,7 @@
 //
 // A stream has only 8 sequential chains, so the GPU codes many streams at
 // once: 8 threads per stream, four streams per warp, a warp per CTA.
+#include "coder.cuh"
 #include "runtime.h"
 #include "../../include/pentago_b200.h"
 #include <cstdint>
@@ -84,22 +85,6 @@ __host__ __device__ inline rans_enc_sym enc_sym(const rans_freq& t, int s) {
     e.bias = t.cum[s];
   }
   return e;
-}
-
-// Selects by a comparison, kept as selects: a predicated instruction waits
-// about 13 cycles for a predicate that a select takes in 4 (measured), and the
-// coders' chains are made of little else.
-// x >= a ? u : v, and the same for a second pair of values
-__device__ __forceinline__ void select_ge(uint32_t x, uint32_t a, uint32_t u0, uint32_t v0, uint32_t& r0, uint32_t u1,
-                                          uint32_t v1, uint32_t& r1) {
-  asm("{\n.reg .pred p;\nsetp.ge.u32 p, %2, %3;\nselp.u32 %0, %4, %5, p;\nselp.u32 %1, %6, %7, p;\n}\n"
-      : "=&r"(r0), "=&r"(r1) : "r"(x), "r"(a), "r"(u0), "r"(v0), "r"(u1), "r"(v1));
-}
-__device__ __forceinline__ uint32_t select_ge(uint32_t x, uint32_t a, uint32_t u, uint32_t v) {
-  uint32_t r;
-  asm("{\n.reg .pred p;\nsetp.ge.u32 p, %1, %2;\nselp.u32 %0, %3, %4, p;\n}\n"
-      : "=r"(r) : "r"(x), "r"(a), "r"(u), "r"(v));
-  return r;
 }
 
 // ---------------------------------------------------------------------------
@@ -393,7 +378,7 @@ rans_encode_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restric
 // The CTA moves len bytes from src down to dst (dst <= src, src + len on a
 // word boundary), whole words at a time.  A round's words are read before any
 // of them is written, and a later round reads above what this one wrote.
-constexpr int kMoveWords = 4;
+constexpr int kPackWords = 4;
 __device__ __forceinline__ void move_down(uint8_t* dst, const uint8_t* src, uint32_t len) {
   if (dst == src) return;
   const uint32_t head = min(len, uint32_t(-reinterpret_cast<uintptr_t>(dst)) & 3u);
@@ -408,17 +393,17 @@ __device__ __forceinline__ void move_down(uint8_t* dst, const uint8_t* src, uint
   const uint32_t sh = 8 * uint32_t(reinterpret_cast<uintptr_t>(src) & 3);
   const uint32_t* from = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(3));
   uint32_t* to = reinterpret_cast<uint32_t*>(dst);
-  for (uint32_t w0 = 0; w0 < words; w0 += kMoveWords * blockDim.x) {
-    uint32_t v[kMoveWords];
+  for (uint32_t w0 = 0; w0 < words; w0 += kPackWords * blockDim.x) {
+    uint32_t v[kPackWords];
 #pragma unroll
-    for (int q = 0; q < kMoveWords; q++) {
+    for (int q = 0; q < kPackWords; q++) {
       const uint32_t w = w0 + q * blockDim.x + threadIdx.x;
       v[q] = 0;
       if (w < words) v[q] = sh ? __funnelshift_r(from[w], from[w + 1], sh) : from[w];
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < kMoveWords; q++) {
+    for (int q = 0; q < kPackWords; q++) {
       const uint32_t w = w0 + q * blockDim.x + threadIdx.x;
       if (w < words) to[w] = v[q];
     }
