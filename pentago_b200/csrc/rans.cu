@@ -5,7 +5,7 @@
 // decode order, header = version(4) | counts(3 x 8) | stream lengths(8 x 4).
 //
 // A stream has only 8 sequential chains, so the GPU codes many streams at
-// once: 8 threads per stream, four streams per warp, a warp per CTA.
+// once: 8 threads per stream, four streams per warp.
 #include "coder.cuh"
 #include "runtime.h"
 #include "../../include/pentago_b200.h"
@@ -90,11 +90,11 @@ __host__ __device__ inline rans_enc_sym enc_sym(const rans_freq& t, int s) {
 // ---------------------------------------------------------------------------
 // Encoding, in three launches:
 //
-//   rans_count_kernel   symbol counts of every stream (the frequency tables),
-//                       over the whole batch at once;
-//   rans_encode_kernel  the coding itself, 8 lanes per stream, each lane's
-//                       bytes at the end of a slot of its own in the output;
-//   rans_pack_kernel    the lanes' bytes moved behind the header.
+//   rans_count_kernel   symbol counts of long streams (the frequency tables);
+//   rans_encode_kernel  the coding itself, 8 lanes per stream, a warp for four
+//                       streams, with the counting and packing of short ones;
+//   rans_pack_kernel    the lanes' bytes of long streams moved from their slots
+//                       to behind the header.
 //
 // The coding is bound by the latency of its 8 chains per stream: a lane's
 // next symbol waits for its last (a compare and select, a multiply-high, a
@@ -104,10 +104,12 @@ __host__ __device__ inline rans_enc_sym enc_sym(const rans_freq& t, int s) {
 // memory a chunk ahead, a symbol's constants are one 16-byte shared load, and
 // the bytes of a renormalization are always written to the lane's buffer,
 // whose position then moves past them or does not; whole words leave it at a
-// chunk's end.  Counting and packing, which 8 lanes did one word or byte at a
-// time, have kernels with the whole chip behind them.  1,024 streams of 1 M symbols of a solved
-// slice: 31.7 ms before, 3.87 ms now (coding 3.56, about 53 cycles a symbol of a
-// lane where the chain itself needs 27, counting 0.18, packing 0.13).
+// chunk's end.  Counting and packing of a long stream have a CTA, as its 8
+// lanes would take as long for them as for the coding; for short ones such
+// CTAs would cost more (14 ns a stream) than the lanes take, and bytes that fit
+// the lanes' buffers never see their slots.  1,024 streams of 1 M symbols:
+// 3.65 ms (coding 3.36, about 53 cycles a symbol of a lane where the chain itself
+// needs 27, counting 0.17, packing 0.11); 65,536 of 512 symbols: 0.12 ms.
 
 constexpr int kChunk = 1024;             // symbols of a stream staged at a time: 128 for each lane
 constexpr int kChunkRow = kChunk + 32;   // the four streams' rows start 8 banks apart
@@ -121,7 +123,7 @@ constexpr uint32_t kOneByteFreq = 64;
 // Ones and twos of a stream, and whether it holds a symbol above 2.
 struct rans_counts {
   uint64_t one, two;
-  uint32_t bad, pad;
+  uint32_t bad;
 };
 
 // Four symbols: ones in the low half of n, twos in the high half.
@@ -130,31 +132,21 @@ __device__ __forceinline__ void count_word(uint32_t w, uint32_t& n, uint32_t& ba
   bad |= (w & 0xfcfcfcfcu) | (w & (w >> 1) & 0x01010101u);
 }
 
-// One CTA per stream: 16-byte loads where the words lie inside the stream,
-// bytes at its ends.  Bound by HBM; a stream of 1 M symbols takes its CTA
-// about 1% of what its chains then take.
-constexpr int kCountThreads = 256;
-__global__ void __launch_bounds__(kCountThreads)
-rans_count_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restrict__ offsets,
-                  const int64_t* __restrict__ expect, rans_counts* __restrict__ counts) {
-  __shared__ uint64_t total[3];
-  const int s = blockIdx.x;
-  const int64_t n = offsets[s + 1] - offsets[s];
-  if (n < 0 || (expect && n != expect[s])) return;   // refused by the encoder
-  if (threadIdx.x < 3) total[threadIdx.x] = 0;
-  __syncthreads();
-  const uint8_t* sym = symbols + offsets[s];
+// The symbols sym[0 .. n) that thread `rank` of TEAM counts: 16-byte loads where the
+// words lie inside the stream, bytes at its ends.  Eight loads are in flight
+// per thread.
+template<int TEAM>
+__device__ __forceinline__ rans_counts count_symbols(const uint8_t* sym, int64_t n, int rank) {
   const int64_t head = min(n, int64_t(-reinterpret_cast<uintptr_t>(sym) & 15)), words = (n - head) >> 4;
   const int64_t tail = head + 16 * words;
   const uint4* W = reinterpret_cast<const uint4*>(sym + head);
-  uint64_t one = 0, two = 0;
-  uint32_t bad = 0;
+  uint32_t one = 0, two = 0, bad = 0;   // (a thread has less than 2^32 of them)
   constexpr int kUnroll = 8;
-  for (int64_t k0 = 0; k0 < words; k0 += kUnroll * kCountThreads) {
+  for (int64_t k0 = 0; k0 < words; k0 += kUnroll * TEAM) {
     uint4 v[kUnroll];
 #pragma unroll
     for (int q = 0; q < kUnroll; q++) {
-      const int64_t k = k0 + q * kCountThreads + threadIdx.x;
+      const int64_t k = k0 + q * TEAM + rank;
       v[q] = k < words ? __ldg(W + k) : make_uint4(0, 0, 0, 0);
     }
     uint32_t m = 0;
@@ -169,22 +161,70 @@ rans_count_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restrict
     two += m >> 16;
   }
   uint32_t m = 0;
-  if (int64_t(threadIdx.x) < head) count_word(sym[threadIdx.x], m, bad);
-  if (int64_t(threadIdx.x) < n - tail) count_word(sym[tail + threadIdx.x], m, bad);
+  for (int i = rank; i < int(head); i += TEAM) count_word(sym[i], m, bad);
+  for (int i = rank; i < int(n - tail); i += TEAM) count_word(sym[tail + i], m, bad);
   one += m & 0xffff;
   two += m >> 16;
-  for (int o = 16; o; o >>= 1) {
-    one += __shfl_xor_sync(0xffffffffu, one, o);
-    two += __shfl_xor_sync(0xffffffffu, two, o);
+  return rans_counts{one, two, bad};
+}
+
+// Streams longer than this, in a batch of nstreams, are left to the kernels of
+// the long ones for their counts and packing.  A few streams have the chip to
+// themselves (64 of 4,096 symbols 42 us with those kernels, 46 without); of many,
+// those that their 8 lanes see to cost less (65,536 of 4,096: 1.24 and 0.42 ms).
+constexpr int64_t kOwnOfFew = 2048, kOwnOfMany = 16384;
+// A CTA of those handles streams blockIdx.x + k gridDim.x: the next 256 of them
+// are looked at together, and f(s, n) called for the long ones, by all threads.
+constexpr int kLongThreads = 256, kLongCtas = 8 * 148;   // (resident at once)
+template<class F>
+__device__ __forceinline__ void each_long(const int64_t* __restrict__ offsets, int nstreams, int64_t own,
+                                          const int64_t* __restrict__ expect, F f) {
+  __shared__ unsigned mask[kLongThreads / 32];
+  for (int64_t k0 = 0; blockIdx.x + k0 * gridDim.x < nstreams; k0 += kLongThreads) {
+    const int64_t s = blockIdx.x + (k0 + threadIdx.x) * gridDim.x;
+    const int64_t n = s < nstreams ? offsets[s + 1] - offsets[s] : 0;
+    const unsigned mine = __ballot_sync(0xffffffffu, n > own && !(expect && n != expect[s]));
+    if ((threadIdx.x & 31) == 0) mask[threadIdx.x >> 5] = mine;
+    __syncthreads();
+    for (int w = 0; w < kLongThreads / 32; w++)
+      for (unsigned left = mask[w]; left; left &= left - 1) {
+        const int64_t t = blockIdx.x + (k0 + 32 * w + __ffs(left) - 1) * gridDim.x;
+        f(t, offsets[t + 1] - offsets[t]);
+      }
+    __syncthreads();
   }
-  bad = __any_sync(0xffffffffu, bad != 0);
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(&total[0]), (unsigned long long)one);
-    atomicAdd(reinterpret_cast<unsigned long long*>(&total[1]), (unsigned long long)two);
-    if (bad) atomicOr(reinterpret_cast<unsigned long long*>(&total[2]), 1ull);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) counts[s] = rans_counts{total[0], total[1], uint32_t(total[2]), 0};
+}
+
+// The counts go into the header of the stream's output, with a version of 0 if
+// the stream cannot be coded.
+__global__ void __launch_bounds__(kLongThreads, 8)
+rans_count_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restrict__ offsets, int nstreams, int64_t own,
+                  const int64_t* __restrict__ expect, uint8_t* __restrict__ out,
+                  const int64_t* __restrict__ out_offsets) {
+  __shared__ unsigned long long total[3];
+  each_long(offsets, nstreams, own, expect, [&](int64_t s, int64_t n) {
+    if (threadIdx.x < 3) total[threadIdx.x] = 0;
+    __syncthreads();
+    rans_counts C = count_symbols<kLongThreads>(symbols + offsets[s], n, threadIdx.x);
+    for (int o = 16; o; o >>= 1) {
+      C.one += __shfl_xor_sync(0xffffffffu, C.one, o);
+      C.two += __shfl_xor_sync(0xffffffffu, C.two, o);
+    }
+    C.bad = __any_sync(0xffffffffu, C.bad != 0);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&total[0], (unsigned long long)C.one);
+      atomicAdd(&total[1], (unsigned long long)C.two);
+      if (C.bad) atomicOr(&total[2], 1ull);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint8_t* base = out + out_offsets[s];
+      put_u32(base, total[2] ? 0 : 2);
+      put_u64(base + 4, uint64_t(n) - total[0] - total[1]);
+      put_u64(base + 12, total[0]);
+      put_u64(base + 20, total[1]);
+    }
+  });
 }
 
 // End of lane l's slot: its bytes are written downward from there in whole
@@ -274,31 +314,49 @@ __device__ __forceinline__ uint4 load_granule(uintptr_t g, uintptr_t a, uintptr_
 }
 
 // One warp, four streams.  out_offsets[s] has room for stream_bound(n_s).
+// (OWN is a constant because it costs 1.5% of the coding as a parameter)
+template<int64_t OWN>
 __global__ void __launch_bounds__(32)
 rans_encode_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restrict__ offsets, int nstreams,
-                   const rans_counts* __restrict__ counts, uint8_t* __restrict__ out,
-                   const int64_t* __restrict__ out_offsets, int64_t* __restrict__ sizes,
+                   uint8_t* out, const int64_t* __restrict__ out_offsets, int64_t* __restrict__ sizes,
                    const int64_t* __restrict__ expect) {
   __shared__ __align__(16) uint8_t stage[kWarpStreams][kChunkRow];
   __shared__ uint4 par[kWarpStreams][3];
   __shared__ __align__(16) uint8_t bytes[32][kLaneRow];
   const int g = threadIdx.x >> 3, lane = threadIdx.x & 7;
-  const int s = blockIdx.x * kWarpStreams + g;
+  const int64_t s = int64_t(blockIdx.x) * kWarpStreams + g;
+  const unsigned group = 0xffu << (8 * g);
   int64_t n = -1;
   uintptr_t a = 0, b = 0;
+  uint8_t* base = nullptr;
   uint64_t c[3] = {0, 0, 0};
   bool frequent = true;   // every symbol that occurs has kOneByteFreq or more
   if (s < nstreams) {
     n = offsets[s + 1] - offsets[s];
     a = reinterpret_cast<uintptr_t>(symbols) + uintptr_t(offsets[s]);
     b = a + uintptr_t(n);
+    base = out + out_offsets[s];
     // With `expect`, a stream of another length has no room reserved: refuse it
-    if (n < 0 || (expect && n != expect[s]) || counts[s].bad) {
+    bool bad = n < 0 || (expect && n != expect[s]);
+    if (!bad && n > OWN) {
+      bad = get_u32(base) != 2;
+      c[1] = get_u64(base + 12);
+      c[2] = get_u64(base + 20);
+    } else if (!bad) {
+      rans_counts C = count_symbols<kLanes>(symbols + offsets[s], n, lane);
+      for (int o = 4; o; o >>= 1) {
+        C.one += __shfl_xor_sync(group, C.one, o, 8);
+        C.two += __shfl_xor_sync(group, C.two, o, 8);
+        C.bad |= __shfl_xor_sync(group, C.bad, o, 8);
+      }
+      bad = C.bad != 0;
+      c[1] = C.one;
+      c[2] = C.two;
+    }
+    if (bad) {
       if (lane == 0) sizes[s] = PG_ERR_ARG;
       n = -1;
     } else {
-      c[1] = counts[s].one;
-      c[2] = counts[s].two;
       c[0] = uint64_t(n) - c[1] - c[2];
       const rans_freq t = make_freq(c);
 #pragma unroll
@@ -315,10 +373,10 @@ rans_encode_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restric
   const uintptr_t first = a & ~uintptr_t(15);
   const int64_t nchunks = n > 0 ? int64_t((b - first + kChunk - 1) / kChunk) : 0;
   const int mine = int((a + lane) & 7);
-  uint8_t* base = n >= 0 ? out + out_offsets[s] : nullptr;
   uint8_t* const buf = bytes[threadIdx.x];
   rans_enc_lane E = {kRansLower, kTop, n >= 0 ? slot_end(base, n, lane) : nullptr};
   uint8_t* const end = E.p;
+  const bool kept = n <= kChunk;   // a lane's bytes all fit its buffer
   constexpr int kGranules = kChunk / 16 / kLanes;
   uint4 next[kGranules];
   auto load_chunk = [&](int64_t k) {
@@ -352,22 +410,39 @@ rans_encode_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restric
         if (one_byte) E.put_chunk<1>(row + mine, P, buf);
         else E.put_chunk<2>(row + mine, P, buf);
       } else {
-        for (int j = kChunk / kLanes - 1; j >= 0; j--) {
+        const int top = b < lo + kChunk ? (int(b - lo) - 1 - mine) >> 3 : kChunk / kLanes - 1;
+        for (int j = top; j >= 0; j--) {
           const uintptr_t at = lo + mine + 8 * j;
-          if (at < a || at >= b) continue;
+          if (at < a) break;
           E.put<2>(P[row[mine + 8 * j]], buf);
         }
       }
-      E.flush(buf);
+      if (!kept) E.flush(buf);
     }
   }
   if (n < 0) return;
-  E.finish(buf);
-  const uint32_t len = uint32_t(end - E.p);
+  if (!kept) E.finish(buf);
+  const uint32_t len = kept ? uint32_t(kTop - E.pos) + 4 : uint32_t(end - E.p);
+  uint64_t upto = len;   // the lanes' up to and with this one
+  for (int o = 1; o < kLanes; o <<= 1) {
+    const uint64_t v = __shfl_up_sync(group, upto, o, 8);
+    if (lane >= o) upto += v;
+  }
+  const uint64_t total = __shfl_sync(group, upto, kLanes - 1, 8);
+  if (kept) {
+    uint8_t* dst = base + kHeader + (upto - len);
+    for (int j = 0; j < 4; j++) dst[j] = uint8_t(E.x >> (24 - 8 * j));
+    for (int k = E.pos; k < kTop; k++) dst[4 + k - E.pos] = buf[k];
+  } else if (n <= OWN) {
+    __syncwarp(group);
+    uint8_t* dst = base + kHeader;
+    for (int l = 0; l < kLanes; l++) {   // (as in rans_pack_kernel)
+      const uint32_t m = __shfl_sync(group, len, l, 8);
+      move_down<kLanes, 8>(dst, slot_end(base, n, l) - m, m, lane, [group] { __syncwarp(group); });
+      dst += m;
+    }
+  }
   put_u32(base + 28 + 4 * lane, len);
-  const unsigned group = 0xffu << (8 * g);
-  uint64_t total = len;
-  for (int o = 4; o; o >>= 1) total += __shfl_xor_sync(group, total, o, 8);
   if (lane == 0) {
     put_u32(base, 2);
     for (int k = 0; k < 3; k++) put_u64(base + 4 + 8 * k, c[k]);
@@ -375,63 +450,22 @@ rans_encode_kernel(const uint8_t* __restrict__ symbols, const int64_t* __restric
   }
 }
 
-// The CTA moves len bytes from src down to dst (dst <= src, src + len on a
-// word boundary), whole words at a time.  A round's words are read before any
-// of them is written, and a later round reads above what this one wrote.
-constexpr int kPackWords = 4;
-__device__ __forceinline__ void move_down(uint8_t* dst, const uint8_t* src, uint32_t len) {
-  if (dst == src) return;
-  const uint32_t head = min(len, uint32_t(-reinterpret_cast<uintptr_t>(dst)) & 3u);
-  const uint32_t words = (len - head) >> 2, tail = len - head - 4 * words;
-  uint8_t hv = 0;
-  if (threadIdx.x < head) hv = src[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x < head) dst[threadIdx.x] = hv;
-  __syncthreads();
-  dst += head;
-  src += head;
-  const uint32_t sh = 8 * uint32_t(reinterpret_cast<uintptr_t>(src) & 3);
-  const uint32_t* from = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(src) & ~uintptr_t(3));
-  uint32_t* to = reinterpret_cast<uint32_t*>(dst);
-  for (uint32_t w0 = 0; w0 < words; w0 += kPackWords * blockDim.x) {
-    uint32_t v[kPackWords];
-#pragma unroll
-    for (int q = 0; q < kPackWords; q++) {
-      const uint32_t w = w0 + q * blockDim.x + threadIdx.x;
-      v[q] = 0;
-      if (w < words) v[q] = sh ? __funnelshift_r(from[w], from[w + 1], sh) : from[w];
+// The lanes' bytes, in lane order, from their slots to behind the header.  A
+// lane's bytes move down, and never past a slot that has not moved yet (they
+// fit their own).
+__global__ void __launch_bounds__(kLongThreads)
+rans_pack_kernel(const int64_t* __restrict__ offsets, int nstreams, int64_t own, const int64_t* __restrict__ expect,
+                 uint8_t* out, const int64_t* __restrict__ out_offsets, const int64_t* __restrict__ sizes) {
+  each_long(offsets, nstreams, own, expect, [&](int64_t s, int64_t n) {
+    if (sizes[s] < 0) return;
+    uint8_t* base = out + out_offsets[s];
+    uint8_t* dst = base + kHeader;
+    for (int l = 0; l < kLanes; l++) {
+      const uint32_t len = get_u32(base + 28 + 4 * l);
+      move_down<kLongThreads, 4>(dst, slot_end(base, n, l) - len, len, threadIdx.x, [] { __syncthreads(); });
+      dst += len;
     }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < kPackWords; q++) {
-      const uint32_t w = w0 + q * blockDim.x + threadIdx.x;
-      if (w < words) to[w] = v[q];
-    }
-    __syncthreads();
-  }
-  uint8_t tv = 0;
-  if (threadIdx.x < tail) tv = src[4 * words + threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x < tail) dst[4 * words + threadIdx.x] = tv;
-  __syncthreads();
-}
-
-// One CTA per stream: the lanes' bytes, in lane order, from their slots to
-// behind the header.  A lane's bytes move down, and never past a slot that
-// has not moved yet (they fit their own).
-__global__ void __launch_bounds__(256)
-rans_pack_kernel(const int64_t* __restrict__ offsets, uint8_t* out,
-                 const int64_t* __restrict__ out_offsets, const int64_t* __restrict__ sizes) {
-  const int s = blockIdx.x;
-  if (sizes[s] < 0) return;
-  const int64_t n = offsets[s + 1] - offsets[s];
-  uint8_t* base = out + out_offsets[s];
-  uint8_t* dst = base + kHeader;
-  for (int l = 0; l < kLanes; l++) {
-    const uint32_t len = get_u32(base + 28 + 4 * l);
-    move_down(dst, slot_end(base, n, l) - len, len);
-    dst += len;
-  }
+  });
 }
 
 // ---------------------------------------------------------------------------
@@ -720,19 +754,25 @@ rans_decode_kernel(const uint8_t* __restrict__ in, const int64_t* __restrict__ i
 
 int64_t rans_stream_bound(int64_t n) { return stream_bound(n); }
 
-int launch_rans_encode(const uint8_t* symbols, const int64_t* offsets, int nstreams, uint8_t* out,
-                       const int64_t* out_offsets, int64_t* sizes, const int64_t* expect, cudaStream_t stream) {
-  stream_scratch scratch(stream);
-  rans_counts* counts = nullptr;
-  PG_CUDA(scratch.alloc(&counts, sizeof(rans_counts) * size_t(nstreams)));
-  rans_count_kernel<<<nstreams, kCountThreads, 0, stream>>>(symbols, offsets, expect, counts);
+template<int64_t OWN>
+static int launch_rans_encoders(const uint8_t* symbols, const int64_t* offsets, int nstreams, uint8_t* out,
+                                const int64_t* out_offsets, int64_t* sizes, const int64_t* expect,
+                                cudaStream_t stream) {
+  const int ctas = nstreams < kLongCtas ? nstreams : kLongCtas;
+  rans_count_kernel<<<ctas, kLongThreads, 0, stream>>>(symbols, offsets, nstreams, OWN, expect, out, out_offsets);
   PG_CUDA(cudaGetLastError());
-  rans_encode_kernel<<<(nstreams + kWarpStreams - 1) / kWarpStreams, 32, 0, stream>>>(
-      symbols, offsets, nstreams, counts, out, out_offsets, sizes, expect);
+  rans_encode_kernel<OWN><<<(nstreams + kWarpStreams - 1) / kWarpStreams, 32, 0, stream>>>(
+      symbols, offsets, nstreams, out, out_offsets, sizes, expect);
   PG_CUDA(cudaGetLastError());
-  rans_pack_kernel<<<nstreams, 256, 0, stream>>>(offsets, out, out_offsets, sizes);
+  rans_pack_kernel<<<ctas, kLongThreads, 0, stream>>>(offsets, nstreams, OWN, expect, out, out_offsets, sizes);
   PG_CUDA(cudaGetLastError());
   return PG_OK;
+}
+
+int launch_rans_encode(const uint8_t* symbols, const int64_t* offsets, int nstreams, uint8_t* out,
+                       const int64_t* out_offsets, int64_t* sizes, const int64_t* expect, cudaStream_t stream) {
+  return (nstreams > 1024 ? launch_rans_encoders<kOwnOfMany> : launch_rans_encoders<kOwnOfFew>)(
+      symbols, offsets, nstreams, out, out_offsets, sizes, expect, stream);
 }
 
 int launch_rans_decode(const uint8_t* in, const int64_t* in_offsets, const int64_t* in_sizes, int nstreams,

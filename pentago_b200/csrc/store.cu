@@ -381,7 +381,8 @@ store_encode_kernel(const uint64_t* __restrict__ nodes, const int64_t* __restric
     for (int l = 0; l < kLanesS; l++) {
       const uint32_t len_l = __shfl_sync(0xffffffffu, len, l);
       const uint32_t dst_l = __shfl_sync(0xffffffffu, before, l);
-      move_down(sbase + kHead + dst_l, sbase + kHead + int64_t(l + 1) * cap - len_l, len_l, lane);
+      move_down<32, 8>(sbase + kHead + dst_l, sbase + kHead + int64_t(l + 1) * cap - len_l, len_l, lane,
+                       [] { __syncwarp(); });
     }
     for (int j = 0; j < 4; j++) sbase[4 * lane + j] = uint8_t(len >> (8 * j));
     if (lane == 0) sizes[b] = kHead + int64_t(total);
