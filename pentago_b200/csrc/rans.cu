@@ -470,16 +470,14 @@ rans_pack_kernel(const int64_t* __restrict__ offsets, int nstreams, int64_t own,
 
 // ---------------------------------------------------------------------------
 // Decoding: one warp, four streams, like the encoder and bound like it by the
-// lanes' chains (symbol, state, renormalization).  What used to lie on the
-// chain and does not any more: a lane's stream bytes, which it took one at a
-// time from global memory when its state ran low, come from a ring in shared
-// memory with the next byte always in a register; the ring is filled by
+// lanes' chains (symbol, state, renormalization).  A lane's stream bytes are
+// not on the chain: they come from a ring in shared memory with the next byte
+// always in a register; the ring is filled by
 // asynchronous copies three blocks ahead, which no register waits for (a
 // warp's 32 lanes run low at different symbols, so a load into a register
 // would stop the warp at nearly every symbol).  Symbols are staged
 // and leave in 16-byte stores.  1,024 streams of 1 M symbols of a solved
-// slice: 20.2 ms before, 3.5 ms now (about 51 cycles a symbol of a lane, 41 of
-// them in block_one).
+// slice: 3.5 ms (about 51 cycles a symbol of a lane, 41 of them in block_one).
 
 constexpr int kBlockSteps = 128;                     // symbols of a lane per block
 constexpr int kBlockSyms = kBlockSteps * kLanes;     // and of a stream
@@ -574,7 +572,90 @@ struct rans_dec_window {
   }
 };
 
-// status[s]: number of symbols decoded, or PG_ERR_FORMAT / PG_ERR_CAPACITY.
+// One lane's part of a stream.  n: its symbols, 0 for a stream that is not decoded.
+struct rans_dec_stream {
+  uint64_t n;
+  rans_freq t;
+  const uint8_t *p, *end, *stream_end;   // the lane's bytes, the stream's end
+  int64_t status;                        // what the stream's is to be
+  bool given;                            // it is to be decoded
+};
+// Header checks as arithmetic_deserialize / arithmetic_decode (arithmetic.cc:403-495).
+__device__ __forceinline__ rans_dec_stream open_stream(const uint8_t* base, int64_t size, int64_t cap, int only_v2,
+                                                       int lane) {
+  rans_dec_stream D = {};
+  // Streams of another version are left to the learned decoder when asked
+  // (whose CTAs that give up say nothing: the status stays this one)
+  if (only_v2 && size >= 4 && get_u32(base) != 2) {
+    D.status = PG_ERR_CUDA;
+    return D;
+  }
+  D.status = PG_ERR_FORMAT;
+  if (size < kHeader || get_u32(base) != 2) return D;
+  uint64_t c[3], total = 0, start = 0;
+  uint32_t mylen = 0;
+  for (int k = 0; k < 3; k++) c[k] = get_u64(base + 4 + 8 * k);
+  const uint64_t n = c[0] + c[1] + c[2];
+  for (int l = 0; l < kLanes; l++) {
+    const uint32_t len = get_u32(base + 28 + 4 * l);
+    if (l < lane) start += len;
+    if (l == lane) mylen = len;
+    total += len;
+  }
+  if (c[0] > n || c[1] > n || c[2] > n || n > ~uint64_t(0) / 0x3fff) return D;
+  if (total != uint64_t(size - kHeader)) return D;
+  D.status = PG_ERR_CAPACITY;
+  if (int64_t(n) > cap) return D;
+  D.status = int64_t(n);
+  D.given = true;
+  D.n = n;
+  D.t = make_freq(c);
+  D.p = base + kHeader + start;
+  D.end = D.p + mylen;
+  D.stream_end = base + size;
+  return D;
+}
+__device__ __forceinline__ rans_dec_table decoder_table(const rans_freq& t) {
+  return rans_dec_table{t.freq[0], t.freq[1], t.freq[2], t.cum[1], t.cum[2]};
+}
+
+// In a batch of more streams than the warps of rans_decode_kernel that are
+// resident at once (its rings leave room for 8 an SM), streams of up to
+// kPlainSymbols are decoded here, byte by byte and by as many warps as fit: 65,536 of 512
+// symbols 74 us (171 there), of 8,192 833 us (1,440), of 16,384 1.96 ms as there.
+// The others get this status for now.
+constexpr int kRingStreams = 8 * 148 * kWarpStreams;
+constexpr int64_t kPlainSymbols = 12288, kLater = INT64_MIN;
+__global__ void __launch_bounds__(256)
+rans_decode_plain_kernel(const uint8_t* __restrict__ in, const int64_t* __restrict__ in_offsets,
+                         const int64_t* __restrict__ in_sizes, int nstreams, uint8_t* __restrict__ symbols,
+                         const int64_t* __restrict__ sym_offsets, const int64_t* __restrict__ sym_caps,
+                         int64_t* __restrict__ status, int only_v2) {
+  const int64_t s = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
+  const int lane = threadIdx.x & 7;
+  if (s >= nstreams) return;
+  const rans_dec_stream D = open_stream(in + in_offsets[s], in_sizes[s], sym_caps[s], only_v2, lane);
+  const bool later = D.n > kPlainSymbols;
+  if (lane == 0) status[s] = later ? kLater : D.status;
+  if (!D.n || later) return;
+  const rans_dec_table F = decoder_table(D.t);
+  const uint8_t* p = D.p;
+  uint32_t x = 0;
+  for (int j = 0; j < 4 && p < D.end; j++) x = x << 8 | *p++;
+  uint8_t* out = symbols + sym_offsets[s];
+  for (int i = lane; i < int(D.n); i += kLanes) {
+    uint32_t v;
+    x = next_symbol(F, x, v);
+    while (x < kRansLower && p < D.end) x = x << 8 | *p++;
+    out[i] = uint8_t(v);
+  }
+}
+
+// Four streams to a warp.  status[s]: number of symbols decoded, or
+// PG_ERR_FORMAT / PG_ERR_CAPACITY.  REST: the streams left by
+// rans_decode_plain_kernel among the kSpan of the CTA.
+constexpr int kSpan = 8;
+template<bool REST>
 __global__ void __launch_bounds__(32)
 rans_decode_kernel(const uint8_t* __restrict__ in, const int64_t* __restrict__ in_offsets,
                    const int64_t* __restrict__ in_sizes, int nstreams, uint8_t* __restrict__ symbols,
@@ -583,173 +664,154 @@ rans_decode_kernel(const uint8_t* __restrict__ in, const int64_t* __restrict__ i
   __shared__ __align__(16) uint8_t ring[32][kRingRow];
   __shared__ __align__(16) uint8_t stage[kWarpStreams][kOutRow];
   const int g = threadIdx.x >> 3, lane = threadIdx.x & 7;
-  const int s = blockIdx.x * kWarpStreams + g;
-  uint64_t n = 0;
-  rans_freq t = {};
-  const uint8_t *p = nullptr, *end = nullptr, *stream_end = nullptr;
-  bool live = s < nstreams;
-  if (live) {
-    const uint8_t* base = in + in_offsets[s];
-    const int64_t size = in_sizes[s];
-    // Streams of another version are left to the learned decoder when asked
-    // (whose CTAs that give up say nothing: the status stays this one)
-    if (only_v2 && size >= 4 && get_u32(base) != 2) {
-      live = false;
-      if (lane == 0) status[s] = PG_ERR_CUDA;
+  int64_t s = int64_t(blockIdx.x) * (REST ? kSpan : kWarpStreams);
+  const int64_t s0 = s;
+  unsigned mask = 0;   // streams s0 + bit that are left
+  if (REST)
+    mask = __ballot_sync(0xffffffffu, threadIdx.x < kSpan && s0 + threadIdx.x < nstreams &&
+                                          status[s0 + threadIdx.x] == kLater);
+  if (REST && !mask) return;
+  do {
+    if (REST) {   // the first four of them
+      unsigned mine = mask;
+      for (int i = 0; i < g; i++) mine &= mine - 1;
+      for (int i = 0; i < kWarpStreams; i++) mask &= mask - 1;
+      s = mine ? s0 + __ffs(mine) - 1 : nstreams;
     } else {
-      // Header checks as arithmetic_deserialize / arithmetic_decode (arithmetic.cc:403-495)
-      int64_t bad = 0;
-      uint64_t c[3] = {0, 0, 0}, total = 0, start = 0;
-      uint32_t mylen = 0;
-      if (size < kHeader || get_u32(base) != 2) {
-        bad = PG_ERR_FORMAT;
-      } else {
-        for (int k = 0; k < 3; k++) c[k] = get_u64(base + 4 + 8 * k);
-        n = c[0] + c[1] + c[2];
-        for (int l = 0; l < kLanes; l++) {
-          const uint32_t len = get_u32(base + 28 + 4 * l);
-          if (l < lane) start += len;
-          if (l == lane) mylen = len;
-          total += len;
-        }
-        if (c[0] > n || c[1] > n || c[2] > n || n > ~uint64_t(0) / 0x3fff) bad = PG_ERR_FORMAT;
-        else if (total != uint64_t(size - kHeader)) bad = PG_ERR_FORMAT;
-        else if (int64_t(n) > sym_caps[s]) bad = PG_ERR_CAPACITY;
-      }
-      if (lane == 0) status[s] = bad ? bad : int64_t(n);
-      if (bad) {
-        live = false;
-      } else {
-        t = make_freq(c);
-        p = base + kHeader + start;
-        end = p + mylen;
-        stream_end = base + size;
-      }
+      s += g;
     }
-  }
-  if (!live) n = 0;
-  uint32_t x = 0;
-  for (int j = 0; j < 4 && p < end; j++) x = (x << 8) | *p++;
-  const rans_dec_table F = {t.freq[0], t.freq[1], t.freq[2], t.cum[1], t.cum[2]};
-  const bool one_byte =
-      __all_sync(0xffffffffu, !n || min(min(F.f0, F.f1), F.f2) >= kOneByteFreq);   // the same for the whole warp
-  // The stream's bytes from the 16-byte boundary at or below p: byte k of
-  // them goes to byte k % kRing of the ring.  The state has taken the first
-  // `taken`; `filled` 16-byte granules have been asked for, and one replaces
-  // only words that are used up.
-  const uintptr_t src = reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15);
-  const int64_t extent = int64_t(reinterpret_cast<uintptr_t>(end) - src);
-  uint8_t* myring = ring[threadIdx.x];
-  int filled = 0;
-  int64_t taken = int64_t(reinterpret_cast<uintptr_t>(p) - src);
-  const int granules = int((extent + 15) / 16);   // (a lane has less than 2^32 bytes)
-  const int whole = int(min(int64_t(granules), int64_t(reinterpret_cast<uintptr_t>(stream_end) - src) / 16));
-  auto top_up = [&]() {
-    const int to = min(int((taken + kRing) >> 4), granules);
-#pragma unroll 1
-    for (; filled < to; filled++) {
-      const int o = (16 * filled) & (kRing - 1);
-      const uint8_t* from = reinterpret_cast<const uint8_t*>(src) + 16 * int64_t(filled);
-      const unsigned at = unsigned(__cvta_generic_to_shared(myring + o));
-      if (filled < whole) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(at), "l"(from) : "memory");
-        if (o < kMirror) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(at + kRing), "l"(from) : "memory");
-      } else {
-        // the last bytes before the stream's end
-        for (int k = 0; from + k < stream_end; k++) {
-          myring[o + k] = from[k];
-          if (o < kMirror) myring[kRing + o + k] = from[k];
-        }
-      }
+    rans_dec_stream D = {};
+    if (s < nstreams) {
+      D = open_stream(in + in_offsets[s], in_sizes[s], sym_caps[s], only_v2, lane);
+      if (lane == 0) status[s] = D.status;
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  rans_dec_window W = {};
-  if (n) {
-    top_up();
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    W.pos = uint32_t(taken) & ~3u;
-    const uint32_t skip = 8 * (uint32_t(taken) & 3);
-    W.hi = __byte_perm(*reinterpret_cast<const uint32_t*>(myring + W.pos), 0, 0x0123) << skip;
-    W.bits = 32 - skip;
-    W.pos += 4;
-    W.nw = __byte_perm(*reinterpret_cast<const uint32_t*>(myring + W.pos), 0, 0x0123);
-  }
-  // Symbols are staged by output address: row byte v of block k is byte
-  // k kBlockSyms + v from the 16-byte boundary at or below the stream's first,
-  // so a block's last `shift` symbols lie past kBlockSyms and move to the
-  // row's start when the rest has left.
-  uint8_t* out = live ? symbols + sym_offsets[s] : nullptr;
-  const int shift = int(reinterpret_cast<uintptr_t>(out) & 15);
-  uint8_t* out0 = out - shift;
-  uint8_t* row = stage[g];
-  const int64_t blocks = int64_t((n + kBlockSyms - 1) / kBlockSyms);
-  const unsigned long long most = __reduce_max_sync(0xffffffffu, unsigned(min(blocks, int64_t(0x7fffffff))));
-  // The fast forms take a block when its lane cannot run out of bytes in it
-  // and the state is a coder's (2^23 .. 2^31, so that no symbol needs a third
-  // byte).  The stream's end, or damage, takes the careful form from there on.
-  const int enough = one_byte ? kBlockSteps : 2 * kBlockSteps;
-  bool careful = false;
-  for (int64_t k = 0; k < int64_t(most); k++) {
-    if (k < blocks) {
-      uint8_t* at = row + shift + lane;
-      careful = careful || extent - taken < enough || x < kRansLower || x >= (1u << 31) ||
-                uint64_t(k + 1) * kBlockSyms > n;
-      if (!careful && one_byte) {
-        top_up();
-        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-        taken += block_one(F, myring + (int(taken) & (kRing - 1)), at, x);
-      } else if (!careful) {
+    const uint64_t n = D.n;
+    const bool live = D.given;
+    const uint8_t *p = D.p, *end = D.end, *stream_end = D.stream_end;
+    uint32_t x = 0;
+    for (int j = 0; j < 4 && p < end; j++) x = (x << 8) | *p++;
+    const rans_dec_table F = decoder_table(D.t);
+    const bool one_byte =
+        __all_sync(0xffffffffu, !n || min(min(F.f0, F.f1), F.f2) >= kOneByteFreq);   // the same for the whole warp
+    // The stream's bytes from the 16-byte boundary at or below p: byte k of
+    // them goes to byte k % kRing of the ring.  The state has taken the first
+    // `taken`; `filled` 16-byte granules have been asked for, and one replaces
+    // only words that are used up.
+    const uintptr_t src = reinterpret_cast<uintptr_t>(p) & ~uintptr_t(15);
+    const int64_t extent = int64_t(reinterpret_cast<uintptr_t>(end) - src);
+    uint8_t* myring = ring[threadIdx.x];
+    int filled = 0;
+    int64_t taken = int64_t(reinterpret_cast<uintptr_t>(p) - src);
+    const int granules = int((extent + 15) / 16);   // (a lane has less than 2^32 bytes)
+    const int whole = int(min(int64_t(granules), int64_t(reinterpret_cast<uintptr_t>(stream_end) - src) / 16));
+    auto top_up = [&]() {
+      const int to = min(int((taken + kRing) >> 4), granules);
 #pragma unroll 1
-        for (int i = 0; i < 2; i++) {
-          top_up();
-          asm volatile("cp.async.wait_group 2;\n" ::: "memory");
-          const uint32_t before = W.pos - (W.bits >> 3);
-          W.half(F, myring, at + 8 * W.kHalf * i, x);
-          taken += W.pos - (W.bits >> 3) - before;
-        }
-      } else {
-        top_up();
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        const int steps = int(min(int64_t(kBlockSteps), (int64_t(n) - k * kBlockSyms - lane + kLanes - 1) / kLanes));
-        for (int j = 0; j < steps; j++) {
-          uint32_t v;
-          x = next_symbol(F, x, v);
-          at[8 * j] = uint8_t(v);
-          while (x < kRansLower && taken < extent) {
-            // (a damaged state can take more in a block than the ring holds)
-            x = x << 8 | (taken < 16 * int64_t(filled) ? myring[taken & (kRing - 1)]
-                                                       : *(reinterpret_cast<const uint8_t*>(src) + taken));
-            taken++;
+      for (; filled < to; filled++) {
+        const int o = (16 * filled) & (kRing - 1);
+        const uint8_t* from = reinterpret_cast<const uint8_t*>(src) + 16 * int64_t(filled);
+        const unsigned at = unsigned(__cvta_generic_to_shared(myring + o));
+        if (filled < whole) {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(at), "l"(from) : "memory");
+          if (o < kMirror) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(at + kRing), "l"(from) : "memory");
+        } else {
+          // the last bytes before the stream's end
+          for (int k = 0; from + k < stream_end; k++) {
+            myring[o + k] = from[k];
+            if (o < kMirror) myring[kRing + o + k] = from[k];
           }
         }
       }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    rans_dec_window W = {};
+    if (n) {
+      top_up();
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      W.pos = uint32_t(taken) & ~3u;
+      const uint32_t skip = 8 * (uint32_t(taken) & 3);
+      W.hi = __byte_perm(*reinterpret_cast<const uint32_t*>(myring + W.pos), 0, 0x0123) << skip;
+      W.bits = 32 - skip;
+      W.pos += 4;
+      W.nw = __byte_perm(*reinterpret_cast<const uint32_t*>(myring + W.pos), 0, 0x0123);
     }
-    __syncwarp();
-    if (k < blocks) {
-      // Row bytes below kBlockSyms are complete (and, after the last block,
-      // those up to the stream's end).  The first block of an unaligned
-      // stream and the last leave by bytes.
-      const int from = k ? 0 : shift;
-      const int stop = k == blocks - 1 ? int(shift + int64_t(n) - k * kBlockSyms) : kBlockSyms;
-      uint8_t* o = out0 + k * kBlockSyms;
-      if (from == 0 && stop == kBlockSyms) {
-        uint4 w[kBlockSyms / 16 / kLanes];
-#pragma unroll
-        for (int i = 0; i < kBlockSyms / 16 / kLanes; i++)
-          w[i] = reinterpret_cast<const uint4*>(row)[lane + kLanes * i];
-#pragma unroll
-        for (int i = 0; i < kBlockSyms / 16 / kLanes; i++) reinterpret_cast<uint4*>(o)[lane + kLanes * i] = w[i];
-      } else {
-        for (int v = 16 * lane; v < stop; v += 16 * kLanes)
-          for (int e = max(v, from); e < min(v + 16, stop); e++) o[e] = row[e];
+    // Symbols are staged by output address: row byte v of block k is byte
+    // k kBlockSyms + v from the 16-byte boundary at or below the stream's first,
+    // so a block's last `shift` symbols lie past kBlockSyms and move to the
+    // row's start when the rest has left.
+    uint8_t* out = live ? symbols + sym_offsets[s] : nullptr;
+    const int shift = int(reinterpret_cast<uintptr_t>(out) & 15);
+    uint8_t* out0 = out - shift;
+    uint8_t* row = stage[g];
+    const int64_t blocks = int64_t((n + kBlockSyms - 1) / kBlockSyms);
+    const unsigned long long most = __reduce_max_sync(0xffffffffu, unsigned(min(blocks, int64_t(0x7fffffff))));
+    // The fast forms take a block when its lane cannot run out of bytes in it
+    // and the state is a coder's (2^23 .. 2^31, so that no symbol needs a third
+    // byte).  The stream's end, or damage, takes the careful form from there on.
+    const int enough = one_byte ? kBlockSteps : 2 * kBlockSteps;
+    bool careful = false;
+    for (int64_t k = 0; k < int64_t(most); k++) {
+      if (k < blocks) {
+        uint8_t* at = row + shift + lane;
+        careful = careful || extent - taken < enough || x < kRansLower || x >= (1u << 31) ||
+                  uint64_t(k + 1) * kBlockSyms > n;
+        if (!careful && one_byte) {
+          top_up();
+          asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+          taken += block_one(F, myring + (int(taken) & (kRing - 1)), at, x);
+        } else if (!careful) {
+#pragma unroll 1
+          for (int i = 0; i < 2; i++) {
+            top_up();
+            asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+            const uint32_t before = W.pos - (W.bits >> 3);
+            W.half(F, myring, at + 8 * W.kHalf * i, x);
+            taken += W.pos - (W.bits >> 3) - before;
+          }
+        } else {
+          top_up();
+          asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+          const int steps = int(min(int64_t(kBlockSteps), (int64_t(n) - k * kBlockSyms - lane + kLanes - 1) / kLanes));
+          for (int j = 0; j < steps; j++) {
+            uint32_t v;
+            x = next_symbol(F, x, v);
+            at[8 * j] = uint8_t(v);
+            while (x < kRansLower && taken < extent) {
+              // (a damaged state can take more in a block than the ring holds)
+              x = x << 8 | (taken < 16 * int64_t(filled) ? myring[taken & (kRing - 1)]
+                                                         : *(reinterpret_cast<const uint8_t*>(src) + taken));
+              taken++;
+            }
+          }
+        }
       }
-      __syncwarp(0xffu << (8 * g));
-      if (lane == 0) *reinterpret_cast<uint4*>(row) = *reinterpret_cast<const uint4*>(row + kBlockSyms);
+      __syncwarp();
+      if (k < blocks) {
+        // Row bytes below kBlockSyms are complete (and, after the last block,
+        // those up to the stream's end).  The first block of an unaligned
+        // stream and the last leave by bytes.
+        const int from = k ? 0 : shift;
+        const int stop = k == blocks - 1 ? int(shift + int64_t(n) - k * kBlockSyms) : kBlockSyms;
+        uint8_t* o = out0 + k * kBlockSyms;
+        if (from == 0 && stop == kBlockSyms) {
+          uint4 w[kBlockSyms / 16 / kLanes];
+#pragma unroll
+          for (int i = 0; i < kBlockSyms / 16 / kLanes; i++)
+            w[i] = reinterpret_cast<const uint4*>(row)[lane + kLanes * i];
+#pragma unroll
+          for (int i = 0; i < kBlockSyms / 16 / kLanes; i++) reinterpret_cast<uint4*>(o)[lane + kLanes * i] = w[i];
+        } else {
+          for (int v = 16 * lane; v < stop; v += 16 * kLanes)
+            for (int e = max(v, from); e < min(v + 16, stop); e++) o[e] = row[e];
+        }
+        __syncwarp(0xffu << (8 * g));
+        if (lane == 0) *reinterpret_cast<uint4*>(row) = *reinterpret_cast<const uint4*>(row + kBlockSyms);
+      }
+      __syncwarp();
     }
-    __syncwarp();
-  }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    if (REST) __syncwarp();
+  } while (REST && mask);
 }
 
 int64_t rans_stream_bound(int64_t n) { return stream_bound(n); }
@@ -778,7 +840,14 @@ int launch_rans_encode(const uint8_t* symbols, const int64_t* offsets, int nstre
 int launch_rans_decode(const uint8_t* in, const int64_t* in_offsets, const int64_t* in_sizes, int nstreams,
                        uint8_t* symbols, const int64_t* sym_offsets, const int64_t* sym_caps, int64_t* status,
                        int only_v2, cudaStream_t stream) {
-  rans_decode_kernel<<<(nstreams + kWarpStreams - 1) / kWarpStreams, 32, 0, stream>>>(
+  const int rest = nstreams > kRingStreams;
+  if (rest) {
+    rans_decode_plain_kernel<<<unsigned((int64_t(nstreams) * kLanes + 255) / 256), 256, 0, stream>>>(
+        in, in_offsets, in_sizes, nstreams, symbols, sym_offsets, sym_caps, status, only_v2);
+    PG_CUDA(cudaGetLastError());
+  }
+  const int each = rest ? kSpan : kWarpStreams;
+  (rest ? rans_decode_kernel<true> : rans_decode_kernel<false>)<<<(nstreams + each - 1) / each, 32, 0, stream>>>(
       in, in_offsets, in_sizes, nstreams, symbols, sym_offsets, sym_caps, status, only_v2);
   PG_CUDA(cudaGetLastError());
   return PG_OK;

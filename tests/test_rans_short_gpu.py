@@ -2,7 +2,8 @@
 lengths where the encoder's and decoder's forms change: the encoder stages
 1,024 symbols at a time and leaves the counting and packing of streams above
 2,048 symbols (16,384 in batches of more than 1,024 streams) to kernels of
-their own; the decoder works in blocks of 1,024.  Streams equal the oracle's
+their own; the decoder works in blocks of 1,024, and streams of up to 12,288
+symbols in batches of more than 4,736 have a kernel of their own.  Streams equal the oracle's
 bytes, decode to the symbols, and write nothing beside their room."""
 import numpy as np
 import pytest
@@ -96,3 +97,37 @@ def test_streams_that_cannot_be_coded(cuda, O, count):
     assert (sz[good] > 0).all()
     for i in good[:40]:
         assert host[at[i]:at[i] + sz[i]].tobytes() == oracle_encode(O, syms[i])
+
+
+@pytest.mark.parametrize("kind", ["rare", "uniform"])
+@pytest.mark.parametrize("damage", ["bytes", "states", "lengths"])
+@pytest.mark.parametrize("others", [0, 4800])
+def test_damaged_streams_in_both_forms(cuda, O, kind, damage, others):
+    """Damage in streams whose symbols need one byte at most and in such that need two, in a few streams and among
+    many: decoded symbol by symbol as the byte-wise rule has it, the streams beside them as they are."""
+    from pentago_b200 import rans
+    rng = np.random.default_rng(len(damage) + others)
+    whole = [draw(rng, 256, kind) for _ in range(40)]
+    good = [oracle_encode(O, s) for s in whole]
+    blobs = [good[i % 40] for i in range(others)]
+    for n in (300, 1500, 6007, 9000, 13000):
+        blob = bytearray(oracle_encode(O, draw(rng, n, kind)))
+        lens = np.frombuffer(bytes(blob[28:60]), "<u4").astype(np.int64)
+        if damage == "bytes":
+            for k in rng.integers(60, len(blob), 20):
+                blob[k] ^= int(rng.integers(1, 256))
+        elif damage == "states":
+            starts = 60 + np.concatenate([[0], np.cumsum(lens)[:-1]])
+            for k, v in zip(starts, (bytes(4), b"\0\0\0\1", b"\0\x7f\xff\xff", b"\xff" * 4, b"\x80\0\0\0")):
+                blob[int(k):int(k) + 4] = v
+        else:
+            lens[0] -= 1
+            lens[1] += 1
+            lens[7] += lens[6] - 2
+            lens[6] = 2
+            blob[28:60] = lens.astype("<u4").tobytes()
+        at = int(rng.integers(0, len(blobs) + 1))
+        blobs.insert(at, bytes(blob))
+    for k, (blob, got) in enumerate(zip(blobs, rans.decode(blobs))):
+        want = [whole[i] for i in range(40) if good[i] is blob] or [decode_bytewise(blob)]
+        assert np.array_equal(got, want[0]), k
