@@ -403,20 +403,18 @@ void carve_scratch(board_plan& P, char* base, bool global_ws) {
 }
 
 // pg_midsolve_batch's scratch: job descriptors, the grid kernel's per-board
-// words, then per larger board its tables and global workspace.  With the
-// caller's scratch, nothing is allocated.  (A shared-memory board needs its
-// descriptor alone; its size here is what callers have been told so far, so
-// that their buffers stay the right ones.)
+// words, then per larger board its tables and global workspace (a
+// shared-memory board needs its descriptor alone).  With the caller's scratch,
+// nothing is allocated.
 static bool smem_board(const board_plan& P) { return P.workspace <= size_t(kSmemWorkspaceMax); }
-static size_t batch_bytes_of(const board_plan& P) { return (smem_board(P) ? 2 : 1) * scratch_bytes_of(P); }
+static size_t batch_bytes_of(const board_plan& P) { return smem_board(P) ? 0 : scratch_bytes_of(P); }
 static size_t small_jobs_bytes(int nsmall) { return align256(sizeof(small_job) * size_t(nsmall)); }
 static size_t jobs_bytes(int nsmall, int nlarge) {
   return small_jobs_bytes(nsmall) + align256(sizeof(mid_job_t) * size_t(nlarge));
 }
 // Everything before the boards' tables.
 static size_t head_bytes(int nsmall, int nlarge) {
-  return align256(624 * size_t(nsmall)) + align256(sizeof(mid_job_t) * 2 * size_t(nsmall)) +
-         align256(sizeof(mid_job_t) * size_t(nlarge)) + (nlarge ? grid_aux_bytes(nlarge) : 0);
+  return jobs_bytes(nsmall, nlarge) + (nlarge ? grid_aux_bytes(nlarge) : 0);
 }
 
 }  // namespace pg
@@ -485,7 +483,7 @@ extern "C" int pg_midsolve_batch(const uint64_t* raws, int n, pg_mid_values_t* o
       small[ns++] = small_job_of(P.job);
     } else {
       carve_scratch(P, base + off);
-      off += scratch_bytes_of(P);
+      off += batch_bytes_of(P);
       large[nl++] = P.job;
     }
   }
