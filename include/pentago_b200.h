@@ -534,6 +534,10 @@ int pg_selftest_midsolve_host(const uint64_t* raws, int n, pg_mid_values_t* out,
 /* The same solve split into `groups` cooperating groups (one host thread
  * each, a shared barrier between levels), as the multi-CTA kernel splits it. */
 int pg_selftest_midsolve_groups_host(const uint64_t* raws, int n, int groups, pg_mid_values_t* out);
+/* The check of the midsolve index tables before they are uploaded, on those of
+ * one count of empty spots (0..10) with `delta` added to one word (what 0: an
+ * item, 1: a child, 2: a subset, 3: a level's place). */
+int pg_selftest_small_tables(int spots, int what, int64_t at, int64_t delta);
 /* A CTA waits at a two-CTA barrier that nobody else reaches, with a limit of
  * `polls` polls: the wait runs out and *fault_out = 1 (device check of the
  * bounded barrier the multi-CTA midsolve and the server use). */

@@ -317,12 +317,43 @@ const small_tables_host& small_tables() {
   return *H;
 }
 
+// Whether every index of one count's tables stays where the pass kernel may go:
+// levels inside the workspace and apart from the level they read, each of
+// their entries written once, children, wins and results that exist.  The
+// kernel relies on it (its indexes are these, whatever the board), where
+// mid_board_body checks each one that it works out.
+static bool small_table_fits(const small_table& T) {
+  const int spots = T.spots, ws = bottleneck(spots);
+  if (spots < 0 || spots > kSmallSpots || ws > kSmemWorkspaceMax || 2 * T.nwins + 1 > kPassWins) return false;
+  auto wins = [&](int n) { return (n < spots ? T.wins[n + 1] : T.nwins) - T.wins[n]; };
+  for (int n = 0; n <= spots; n++) {
+    const int items = T.items[n];
+    if (T.wins[n] < 0 || wins(n) < 0 || T.lo[n] < 0 || items < 0 || T.lo[n] + items > ws) return false;
+    if (n < spots && T.lo[n] < T.lo[n + 1] + T.items[n + 1] && T.lo[n + 1] < T.lo[n] + items) return false;
+    if (n <= 1 && n + items > spots + 1) return false;
+    std::vector<bool> written(items, false);
+    for (int it = 0; it < items; it++) {
+      const uint32_t rec = T.recs[T.rec[n] + it];
+      const int o = int(rec & 8191), s0 = int(rec >> 13 & 255), s1 = int(rec >> 21);
+      if (o >= items || written[o] || s1 >= wins(n) || s0 >= (n ? wins(n - 1) : 1)) return false;
+      written[o] = true;
+      for (int c = 0; c < spots - n; c++)
+        if (T.children[T.child[n] + size_t(c) * items + it] >= T.items[n + 1]) return false;
+    }
+  }
+  for (int x = 0; x < T.nwins; x++)
+    if ((T.subsets[x] >> 10) > spots || (T.subsets[x] & 1023) >= 1 << spots) return false;
+  return true;
+}
+
 // Their copies on each device.
 static small_table* small_dev[64];
 static int upload_small_tables() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return PG_ERR_CUDA;
   const small_tables_host& H = small_tables();
+  for (const small_table& T : H.table)
+    if (!small_table_fits(T)) return PG_ERR_BOUNDS;
   uint32_t* recs = nullptr;
   uint16_t *children = nullptr, *subsets = nullptr;
   small_table* tables = nullptr;
@@ -526,6 +557,31 @@ extern "C" int pg_debug_barrier_timeout(unsigned polls, int* fault_out) {
   PG_CUDA(cudaMemcpyAsync(fault_out, fault, sizeof(int), cudaMemcpyDeviceToHost, st));
   PG_CUDA(cudaStreamSynchronize(st));
   return PG_OK;
+}
+
+// The check of the index tables, of one count of empty spots with one word
+// changed (what 0: items' words, 1: children, 2: the wins' subsets, 3: where a
+// level lies; delta 0: as they are).  PG_OK, or PG_ERR_BOUNDS if it refuses them.
+extern "C" int pg_selftest_small_tables(int spots, int what, int64_t at, int64_t delta) {
+  if (spots < 0 || spots > kSmallSpots || what < 0 || what > 3) return fail(PG_ERR_ARG, "bad arguments");
+  small_table T = small_tables().table[spots];
+  size_t items = 0, children = 0;
+  for (int n = 0; n <= spots; n++) {
+    items += T.items[n];
+    children += size_t(T.items[n]) * size_t(spots - n);
+  }
+  std::vector<uint32_t> recs(T.recs, T.recs + items);
+  std::vector<uint16_t> kids(T.children, T.children + children), subsets(T.subsets, T.subsets + T.nwins);
+  const size_t sizes[4] = {recs.size(), kids.size(), subsets.size(), size_t(spots + 1)};
+  if (at < 0 || size_t(at) >= sizes[what]) return fail(PG_ERR_ARG, "no such word");
+  if (what == 0) recs[at] += uint32_t(delta);
+  if (what == 1) kids[at] = uint16_t(kids[at] + delta);
+  if (what == 2) subsets[at] = uint16_t(subsets[at] + delta);
+  if (what == 3) T.lo[at] += int(delta);
+  T.recs = recs.data();
+  T.children = kids.data();
+  T.subsets = subsets.data();
+  return small_table_fits(T) ? PG_OK : fail(PG_ERR_BOUNDS, "an index leaves its table");
 }
 
 // The kernel's own solve, run single-threaded on the host (CPU self-test of
