@@ -534,6 +534,9 @@ int pg_selftest_midsolve_host(const uint64_t* raws, int n, pg_mid_values_t* out,
 /* The same solve split into `groups` cooperating groups (one host thread
  * each, a shared barrier between levels), as the multi-CTA kernel splits it. */
 int pg_selftest_midsolve_groups_host(const uint64_t* raws, int n, int groups, pg_mid_values_t* out);
+/* A per-device set-up that fails `failures` times, called failures + 2 times:
+ * *runs = how often it ran; returns the last call's result. */
+int pg_selftest_once(int failures, int* runs);
 /* The check of the midsolve index tables before they are uploaded, on those of
  * one count of empty spots (0..10) with `delta` added to one word (what 0: an
  * item, 1: a child, 2: a subset, 3: a level's place). */

@@ -139,6 +139,7 @@ SIGNATURES = {
     "pg_midsolve_workspace_size": (_I, [_I]),
     "pg_selftest_midsolve_host": (_I, [_P, _I, _P, _P]),
     "pg_selftest_midsolve_groups_host": (_I, [_P, _I, _I, _P]),
+    "pg_selftest_once": (_I, [_I, ctypes.POINTER(_I)]),
     "pg_selftest_small_tables": (_I, [_I, _I, _I64, _I64]),
     "pg_debug_learned_encode": (_I, [_P, _P, _I, _P, _P, _P, _P, _P, _P]),
     "pg_debug_learned_decode": (_I, [_P, _P, _I, _P, _P, _P, _P, _P, _P, _P, _P]),

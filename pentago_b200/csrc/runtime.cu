@@ -2,8 +2,9 @@
 #include "runtime.h"
 #include "tables.h"
 #include "../../include/pentago_b200.h"
-#include <map>
+#include <atomic>
 #include <mutex>
+#include <set>
 #include <vector>
 
 namespace pg {
@@ -18,17 +19,21 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 static std::mutex once_mutex;
-static std::map<std::pair<int, const void*>, int> once_done;
+static std::set<std::pair<int, const void*>> once_done;
+
+static int once_on(int dev, const void* key, int (*f)()) {
+  std::lock_guard<std::mutex> lock(once_mutex);
+  if (once_done.count({dev, key})) return PG_OK;
+  const int rc = f();
+  if (rc == PG_OK) once_done.insert({dev, key});
+  else (void)cudaGetLastError();   // (reported by rc: not the next launch's)
+  return rc;
+}
 
 int per_device_once(const void* key, int (*f)()) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return fail(PG_ERR_CUDA, "no CUDA device");
-  std::lock_guard<std::mutex> lock(once_mutex);
-  auto it = once_done.find({dev, key});
-  if (it != once_done.end()) return it->second;
-  const int rc = f();
-  once_done[{dev, key}] = rc;
-  return rc;
+  return once_on(dev, key, f);
 }
 
 static std::mutex dev_mutex;
@@ -121,4 +126,19 @@ extern "C" const void* pg_selftest_table(const char* name, int* bytes) {
   if (n == "rotation_minimal_quadrants_flat") { *bytes = 2 * T.rmin_count; return T.rmin_flat; }
   *bytes = 0;
   return nullptr;
+}
+
+// per_device_once of a set-up that fails `failures` times, run failures + 2
+// times: *runs = how often the set-up ran; returns the last call's result.
+static thread_local int once_failures, once_runs;
+static int failing_setup() { return once_runs++ < once_failures ? PG_ERR_CUDA : PG_OK; }
+extern "C" int pg_selftest_once(int failures, int* runs) {
+  static std::atomic<char*> key{nullptr};   // (no address: each call another)
+  const void* k = key.fetch_add(1);
+  once_failures = failures;
+  once_runs = 0;
+  int rc = PG_ERR_ARG;
+  for (int i = 0; i < failures + 2; i++) rc = pg::once_on(-1, k, failing_setup);
+  *runs = once_runs;
+  return rc;
 }

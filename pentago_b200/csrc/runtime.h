@@ -37,9 +37,10 @@ const dev_tables_t* device_tables();
 // arithmetic on the CPU.
 dev_tables_t host_tables_view();
 
-// Run f() once per (current device, key) and return its result from then on
-// (thread safe).  For per-device set-up such as kernel attributes and
-// constant-memory uploads.
+// Run f() once per (current device, key) (thread safe): PG_OK from then on once
+// it has succeeded, while a set-up that failed, for want of memory say, is
+// tried again by the next call.  For per-device set-up such as kernel attributes
+// and constant-memory uploads.
 int per_device_once(const void* key, int (*f)());
 
 // Device scratch of one call: allocated with cudaMallocAsync on the call's
