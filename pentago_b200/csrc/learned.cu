@@ -1704,6 +1704,7 @@ static int learned_encode(const uint8_t* model, const pg_block_ref_t* blocks, in
                           int64_t* sizes, void* stream) {
   if (nstreams < 0 || (nstreams && !blocks)) return fail(PG_ERR_ARG, "bad stream list");
   if (!nstreams) return PG_OK;
+  if (!model) return fail(PG_ERR_ARG, "null model");
   const cudaStream_t st = (cudaStream_t)stream;
   const dev_tables_t* T = device_tables();
   if (!T) return PG_ERR_CUDA;
@@ -1740,6 +1741,7 @@ static int learned_decode(const uint8_t* model, const pg_block_ref_t* blocks, in
                           const int64_t* sym_offsets, const int64_t* sym_caps, int64_t* status, void* stream) {
   if (nstreams < 0 || (nstreams && !blocks)) return fail(PG_ERR_ARG, "bad stream list");
   if (!nstreams) return PG_OK;
+  if (!model) return fail(PG_ERR_ARG, "null model");
   const cudaStream_t st = (cudaStream_t)stream;
   const dev_tables_t* T = device_tables();
   if (!T) return PG_ERR_CUDA;
@@ -1790,6 +1792,7 @@ extern "C" int pg_learned_freqs(const uint8_t* model, const pg_block_ref_t* bloc
                                 uint32_t* freqs, void* stream) {
   if (nstreams < 0 || n < 0 || (nstreams && !blocks)) return fail(PG_ERR_ARG, "bad arguments");
   if (!n) return PG_OK;
+  if (!model) return fail(PG_ERR_ARG, "null model");
   const cudaStream_t st = (cudaStream_t)stream;
   const dev_tables_t* T = device_tables();
   if (!T) return PG_ERR_CUDA;
