@@ -508,9 +508,9 @@ PG_HD void child_half(const line_dev_t& L, const microline_geom& geom, const uin
 // (about 80% of the cycles).  Each pair of threads therefore trades halves and
 // writes its two nodes one after the other, both halves at once: half as many
 // lines per access, and as many for what is read back when accumulating.
-// Lines of axis 0 of a sweep of 59 M parents: 2.42 ms before, 2.09 now.  On
-// axis 3, where the nodes of a line are neighbours, the trade costs more than
-// it saves (2.48 and 2.59 ms), and each thread writes its own node.
+// Lines of axis 0 of a sweep of 59 M parents: 2.09 ms, 2.42 with each thread
+// writing its own node.  On axis 3, where the nodes of a line are neighbours, the
+// trade costs more than it saves (2.59 and 2.48 ms), and each does.
 template<int DIM>
 PG_HD void parent_node(const line_dev_t& L, const microline_geom& G, const uint2* tab0, const uint4* qs,
                        const uint2* pats, const uint4 h, const uint4* rec, int i, bool real, unsigned mask,

@@ -348,9 +348,9 @@ __device__ __forceinline__ uint32_t lm_act_q2(float a, float s, float b, float t
 // Bound by the instructions of a step, 1,700 a warp, and their chain: 7,500
 // cycles for three warps a scheduler, of which the operands take 900, the
 // products 700 each, activations 900, layer 3 1,300, the frequencies 1,000 and the
-// states 700.  2,048 blocks of a solved slice: 166 ms each way with mma.sync
+// states 700.  2,048 blocks of a solved slice: 75 ms each way; 166 with mma.sync
 // (256 products a step and stream), 87 with two warps per stream, one tile
-// and the operands in tensor memory (6 streams an SM instead of 12), 75 now.
+// and the operands in tensor memory (6 streams an SM instead of 12).
 constexpr int kLmCodeThreads = 128;
 constexpr int kLmRowWords = 17;
 constexpr int kLmWordWin = 512;   // the decoder's window of upcoming stream words
@@ -977,17 +977,22 @@ __global__ void lm_choose_kernel(uint8_t* __restrict__ out, const int64_t* __res
 // ---------------------------------------------------------------------------
 // Training
 
-// One CTA takes tiles of 224 samples, a warp 16 of them (a batch of 32,768
-// is then one tile for each of 147 SMs).  Every product runs on the tensor
+// One CTA takes tiles of 224 samples, a warp 16 of them: the largest tile whose
+// features, activations and terms fit shared memory beside the weights, as a tile
+// costs its barriers and the products over samples whatever it holds.  A batch
+// takes the time of its fullest SM: one tile up to 33,152 samples (40 us),
+// two from there on.  Every product runs on the tensor
 // cores (mma.sync m16n8k16, bf16 inputs, fp32 accumulation): the one-hot
 // features, the coding weights and the activations hq / 16 are exact in bf16,
 // and the fp32 gradients dL/da2 and dL/da1 enter as three bf16 terms that add
-// up to them exactly, so no product is rounded and sums are fp32 as before.
-// A warp keeps its 16 samples in registers from layer 1 to dL/da1; the
-// features, activations and gradient terms also lie in shared memory, where
-// the products over samples (dW1, dW2) read them transposed.  Batch 32,768:
-// 910 us with one thread per sample and fp32 loops over shared memory, 40 us
-// now; its error against 64 bits is 2.6e-7 of the gradient (4.0e-7 before).
+// up to them exactly, so no product is rounded; the products of a step of 16
+// samples are summed by the tensor cores and join the rest by rounded fp32
+// additions (add_part).  A warp keeps its 16 samples in registers from layer 1
+// to dL/da1; the features, activations and gradient terms also lie in shared
+// memory, where the products over samples (dW1, dW2) read them transposed.  The
+// error against 64 bits is 0.7e-7 of the gradient's norm; one thread per sample
+// and fp32 loops over shared memory take 910 us for a batch of 32,768 and have
+// 1.0e-7 to 2.1e-7.
 constexpr int kGradWarps = 14;
 constexpr int kGradThreads = 32 * kGradWarps;
 constexpr int kTile = 16 * kGradWarps;
@@ -1503,8 +1508,8 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
 }
 
 // The CTAs' partial sums, added in a fixed order: eight threads to a
-// parameter, each an eighth of the CTAs, then the eight (5.8 us with one thread
-// to a parameter, 3.7 us now).
+// parameter, each an eighth of the CTAs, then the eight: 3.7 us (5.8 with one
+// thread to a parameter).
 constexpr int kReduceParts = 8;
 __global__ void __launch_bounds__(256)
 lm_reduce_kernel(const float* __restrict__ partial, int nparts, float* __restrict__ grad, float* __restrict__ loss) {

@@ -66,7 +66,7 @@ mid_board_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict_
   uint4* ws = SMEM ? smem + tile_bytes / sizeof(uint4) : J.workspace;
   const mid_tables MT = {choose.row, c_winpat, wf};
   mid_board_body(J, MT, reinterpret_cast<char*>(smem), ws, raw, &fault, threadIdx.x, blockDim.x, 0, 1, sync_threads(),
-                 sync_threads(), nullptr, 0, 2, true, tile_bytes);
+                 sync_threads(), nullptr, tile_bytes);
 }
 
 // The boards of pg_midsolve_batch whose workspace fits shared memory: a
@@ -76,8 +76,12 @@ mid_board_kernel(const mid_job_t* __restrict__ jobs, const uint32_t* __restrict_
 // until CTA 0 has the results of both and writes the records.  Bound by
 // the items: integer instructions (rmax, at half rate), conflicts of the
 // gathers from shared memory, and 11 barriers, about evenly.  64 boards of
-// 26 stones: 97 us with the indexes worked out by each CTA, 38 us now (passes
-// 28, wins 5; 512 and 1,024 threads within 2 us of this).
+// 26 stones: 38 us (passes 28, wins 5; 512 and 1,024 threads within 2 us of
+// this; 97 us with the indexes worked out by each CTA, mid_board_body).  The
+// server and the call that must not allocate solve such boards with
+// mid_board_body all the same: a worker of the server is one CTA of 256 threads
+// with 24 KB of shared memory beside others that solve larger boards, and the
+// tables are allocated.
 __global__ void __cluster_dims__(2) __launch_bounds__(kPassThreads)
 mid_pass_kernel(const small_job* __restrict__ jobs, const uint32_t* __restrict__ wf,
                 const small_table* __restrict__ tables) {

@@ -443,28 +443,25 @@ __device__ void traverse_warps(const uint64_t* root, uint32_t ply, const uint64_
 // The whole solve of one board by ncta groups of nt cooperating threads
 // (thread tid of group cta).  `barrier` synchronizes one group, `gbarrier`
 // all groups (with one group it is the same barrier).  Inside a level the
-// (s0, s1p) items are split into one contiguous range per group, and each
-// group builds the set0 rows of its own range; a level's output is read by
-// the next level only after the all-group barrier.  Run with one group of one
-// thread and no-op barriers it is the same computation done sequentially
-// (used by the CPU self-test).  `raw` and `fault` are shared by the groups.
-// Passes [pass0, pass1) are run (the two passes share nothing but the
-// per-level tables); `finish` = false stops after them, leaving the records
-// to a caller that gathers both passes' raw results.  `tile` has room for
-// tile_bytes of s0 rows.
+// (s0, s1p) items are split into contiguous chunks dealt out to the groups in
+// turn, and each group builds the rows of its own chunks; a level's output is
+// read by the next level only after the all-group barrier.  Run with one group
+// of one thread and no-op barriers it is the same computation done sequentially
+// (used by the CPU self-test).  `raw` and `fault` are shared by the groups;
+// `tile` has room for tile_bytes of s0 rows.
 //
 // Bound by the instructions of a level's items and, on small boards, by the
 // chain of levels, so what an item needs is laid out beforehand: the stones of
 // its s1p (5 bits each, and as a mask above them) in one word, the two sums
 // over them in one table word per stone, the children's columns side by side
-// for neighbouring s1p, and a row's table built by one thread per entry.
-// 64 boards of 26 stones: 242 us before, 97 us now; a board of 18 stones:
-// 12.0 ms before, 5.9 ms now.
+// for neighbouring s1p, and a row's table built by one thread per entry.  A
+// board of 18 stones on all SMs: 5.8 ms (12.0 with the indexes worked out from
+// each item's subsets); 64 boards of 26 stones, a CTA each: 0.25 ms with what the
+// call costs (0.51).
 template<class Barrier, class GridBarrier>
 PG_HD void mid_board_body(const mid_job_t& J, const mid_tables& MT, char* tile, uint4* ws,
                           uint4 (*raw)[19], int* fault, int tid, int nt, int cta, int ncta, Barrier barrier,
-                          GridBarrier gbarrier, uint4* dump = nullptr, int pass0 = 0, int pass1 = 2,
-                          bool finish = true, int tile_bytes = kTileBytes) {
+                          GridBarrier gbarrier, uint4* dump = nullptr, int tile_bytes = kTileBytes) {
   const int spots = J.spots;
   const int gtid = cta * nt + tid, gnt = ncta * nt;
   // Per-level tables, the same for both passes (midengine.cc:57-76, :101-107),
@@ -507,7 +504,7 @@ PG_HD void mid_board_body(const mid_job_t& J, const mid_tables& MT, char* tile, 
   }
   gbarrier();
 
-  for (int aggressive = pass0; aggressive < pass1; aggressive++) {
+  for (int aggressive = 0; aggressive < 2; aggressive++) {
     for (int n = spots; n >= 0; n--) {
       const level_t L = make_level(J, MT, n);
       const mid_grab gi = J.spaces[n + 1], go = J.spaces[n];
@@ -548,7 +545,6 @@ PG_HD void mid_board_body(const mid_job_t& J, const mid_tables& MT, char* tile, 
     }
   }
 
-  if (!finish) return;
   // Interleave (midengine.cc:119-124) and traverse; a failed bounds check
   // marks the record with size -1 instead.
   if (gtid == 0 && *fault) { J.out->size = -1; J.out->pad = 0; }

@@ -288,9 +288,10 @@ shard_linear_kernel(const shard_dev_t D, const block_dev_t* __restrict__ blocks,
 // Entries of shards lo .. hi - 1 in order, 256 a warp and turn (8 a thread, so
 // that 8 lookups are in flight; 16 are no faster).  Bound by the lookups,
 // sectors of 32 bytes at random places of n / 4 bytes.  Slice 9 into 1,024
-// shards (3.55 G entries, 0.9 GB of them): 69 ms by bytes, 58.5 ms now
-// (59 G lookups/s) and 4 to 8 ms for the call's scratch to be mapped; slice 7
-// (in L2): 3.6 and 0.8 ms (180 G/s); one shard of slice 9: 12.9 and 2.8 ms.
+// shards (3.55 G entries, 0.9 GB of them): the kernels take 58.5 ms (59 G
+// lookups/s), the call 61 to 69, as its scratch has to be mapped (shard_scatter_kernel
+// 70); slice 7 (in L2): 0.8 ms (180 G/s) and 3.6; one shard of slice 9: 2.8 and
+// 12.9 ms.
 constexpr int kGather = 8;
 template<class U> __global__ void __launch_bounds__(256)
 shard_gather_kernel(const perm_t P, const uint32_t* __restrict__ linear, int shift, int lo, int hi, int64_t total,

@@ -162,8 +162,8 @@ struct word_index {
 // itself).  Bound by the shared-memory counters: most symbols of a solved
 // slice fall on a few of them, and a warp's additions to one address go one
 // after another, so there are kCopies of each counter, used by different
-// lanes.  2,000 blocks: 4.9 ms with one copy and two barriers a node, 1.3 ms
-// now.
+// lanes.  2,000 blocks: 1.3 ms (4.9 with one copy, a thread per rotation and two
+// barriers a node).
 constexpr int kCopies = 8;
 constexpr size_t kHistSmem = sizeof(unsigned) * 4 * kCtx * kCopies;
 __global__ void __launch_bounds__(kThreads)
@@ -231,7 +231,7 @@ __global__ void store_table_kernel(const unsigned* __restrict__ hist, uint16_t* 
 // and symbol is one 16-byte shared load (64 KB of tables, once per SM: hence
 // one CTA of 1,024 threads), a renormalization is selects, and its bytes
 // gather in a register and leave as whole words.  17.6 M nodes (6,000 blocks)
-// of a solved slice: 17.1 ms before, 6.6 ms now (30 instructions a symbol, 20 of
+// of a solved slice: 6.6 ms (30 instructions a symbol, 20 of
 // them on the ALU pipe).
 
 // {xmax, rcp, bias, shift | cmpl << 5} of context c and symbol v at
@@ -400,8 +400,8 @@ store_encode_kernel(const uint64_t* __restrict__ nodes, const int64_t* __restric
 // words give is made for 16 symbols at once.  The next 32 stream bits are
 // picked from a ring in shared memory before every two symbols (which take at
 // most that many); the ring's words lie in the thread's column and come by
-// asynchronous copies, eight symbols ahead.  17.6 M nodes: 17.3 ms before, 6.6 ms
-// now (36 instructions a symbol, 22 on the ALU pipe).
+// asynchronous copies, eight symbols ahead.  17.6 M nodes: 6.6 ms
+// (36 instructions a symbol, 22 on the ALU pipe).
 
 constexpr int kRing = 16;   // words of a lane's ring; row kRing repeats row 0
 constexpr int kDecTable = 5 * kCtx;   // words of the tables
