@@ -1039,28 +1039,42 @@ template<int ROW> __device__ __forceinline__ void frag_bn(uint32_t* b, const uin
 }
 
 // v = term 0 + term 1 + term 2, bf16 each, exactly (8 bits of v's 24 each),
-// for two values packed per word.  Of a value that rounds to an infinity the
-// first term is cut instead; of an infinity or NaN it is that, the others 0.
-__device__ __noinline__ uint32_t split_odd(float v) {
-  const uint32_t u = f_raw(v);
-  return (u & 0x7fffffffu) >= 0x7f7f8000u ? u >> 16 | (v == v ? 0u : 0x40u) : uint32_t(bf16_round_number(v));
+// for two values packed per word; |v| < kSplitMost.
+constexpr float kSplitMost = 3.38e38f;   // (what is not below may round to an infinity)
+__device__ __forceinline__ uint32_t bf16_pair(float v0, float v1) {   // rounded to nearest even; NaN stays NaN
+  uint32_t d;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(v1), "f"(v0));
+  return d;
 }
 __device__ __forceinline__ void split3(float v0, float v1, uint32_t* term) {
-  term[0] = uint32_t(bf16_round_number(v0)) | uint32_t(bf16_round_number(v1)) << 16;
-  float r0 = f_add(v0, -f_bits(term[0] << 16)), r1 = f_add(v1, -f_bits(term[0] & 0xffff0000u)), most;
-  asm("max.NaN.f32 %0, %1, %2;" : "=f"(most) : "f"(fabsf(v0)), "f"(fabsf(v1)));
-  if (!(most < 3.38e38f)) {
-    term[0] = split_odd(v0) | split_odd(v1) << 16;
-    r0 = f_finite(v0) ? f_add(v0, -f_bits(term[0] << 16)) : 0.f;
-    r1 = f_finite(v1) ? f_add(v1, -f_bits(term[0] & 0xffff0000u)) : 0.f;
-  }
 #pragma unroll
-  for (int s = 1; s < 3; s++) {
-    const uint16_t a = bf16_round_number(r0), b = bf16_round_number(r1);
-    term[s] = uint32_t(a) | uint32_t(b) << 16;
-    r0 = f_add(r0, -bf16_value(a));
-    r1 = f_add(r1, -bf16_value(b));
+  for (int s = 0; s < 3; s++) {
+    term[s] = bf16_pair(v0, v1);
+    v0 = f_add(v0, -f_bits(term[s] << 16));
+    v1 = f_add(v1, -f_bits(term[s] & 0xffff0000u));
   }
+}
+// The same of any values: of a large one the first term is cut, of an infinity or
+// NaN it is that and the others 0.
+__device__ __forceinline__ float split_first(float v, float& rest) {
+  const uint32_t u = f_raw(v) & 0xffff0000u;
+  const float first = v == v ? f_bits(u) : f_bits(0x7fff0000u);
+  rest = f_finite(v) ? f_add(v, -first) : 0.f;
+  return first;
+}
+__device__ __forceinline__ void split3_any(float v0, float v1, uint32_t* term) {
+  float r0, r1;
+  const float f0 = split_first(v0, r0), f1 = split_first(v1, r1);
+  term[0] = f_raw(f0) >> 16 | (f_raw(f1) & 0xffff0000u);
+  uint32_t more[3];
+  split3(r0, r1, more);   // (16 bits are left: two terms)
+  term[1] = more[0];
+  term[2] = more[1];
+}
+__device__ __forceinline__ float most_of(float m, float v) {   // max(m, |v|), NaN if either is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(m), "f"(fabsf(v)));
+  return d;
 }
 
 // The coding weights in bf16: stone rows and biases rounded, W1's rotation,
@@ -1346,34 +1360,50 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
       }
     }
     // dW3, and dL/da2 in its terms
+    auto d2_at = [&](int nt, int half, int e) {
+      const float4 w3 = *reinterpret_cast<const float4*>(G.w3[8 * nt + 2 * t + e]);
+      return acc[nt][2 * half + e] > 0.f ? w3.x * dz[half][0] + w3.y * dz[half][1] + w3.z * dz[half][2] : 0.f;
+    };
+    auto put_terms = [&](int nt, int half, const uint32_t* w) {
+#pragma unroll
+      for (int s = 0; s < 3; s++) *reinterpret_cast<uint32_t*>(&G.d[s][row0 + g + 8 * half][8 * nt + 2 * t]) = w[s];
+    };
+    float most = 0.f;
 #pragma unroll
     for (int nt = 0; nt < 8; nt++) {
-      float d[2][2];
 #pragma unroll
       for (int e = 0; e < 2; e++) {
-        const int j = 8 * nt + 2 * t + e;
-        const float4 w3 = *reinterpret_cast<const float4*>(G.w3[j]);
         float v[3] = {};
 #pragma unroll
         for (int half = 0; half < 2; half++) {
-          const float a2 = acc[nt][2 * half + e], r = relu(a2);
+          const float r = relu(acc[nt][2 * half + e]);
 #pragma unroll
           for (int c = 0; c < 3; c++) v[c] = fmaf(r, dz[half][c], v[c]);
-          d[half][e] = a2 > 0.f ? w3.x * dz[half][0] + w3.y * dz[half][1] + w3.z * dz[half][2] : 0.f;
         }
 #pragma unroll
         for (int c = 0; c < 3; c++) {
           v[c] = over_quads(v[c]);
-          if (g == 0) G.gw3[warp][c][j] += v[c];
+          if (g == 0) G.gw3[warp][c][8 * nt + 2 * t + e] += v[c];
         }
       }
 #pragma unroll
       for (int half = 0; half < 2; half++) {
+        const float d0 = d2_at(nt, half, 0), d1 = d2_at(nt, half, 1);
+        most = most_of(most_of(most, d0), d1);
         uint32_t w[3];
-        split3(d[half][0], d[half][1], w);
-#pragma unroll
-        for (int s = 0; s < 3; s++) *reinterpret_cast<uint32_t*>(&G.d[s][row0 + g + 8 * half][8 * nt + 2 * t]) = w[s];
+        split3(d0, d1, w);
+        put_terms(nt, half, w);
       }
+    }
+    if (!(most < kSplitMost)) {
+#pragma unroll
+      for (int nt = 0; nt < 8; nt++)
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+          uint32_t w[3];
+          split3_any(d2_at(nt, half, 0), d2_at(nt, half, 1), w);
+          put_terms(nt, half, w);
+        }
     }
     __syncwarp();
     // dL/da1 = dL/da2 W2^T where the quantizer passes the gradient straight
@@ -1417,12 +1447,22 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
       if (unit < 16) sample_product(g2[u], G.h, G.d, 16 * (unit >> 2), 16 * (unit & 3), lane);
       else if (unit < kUnits2) sample_product(g2[u], G.x, G.d, 112, 16 * (unit & 3), lane);
     }
-    float probe = 0.f;   // 0 if they are all finite
+    most = 0.f;
 #pragma unroll
     for (int nt = 0; nt < 8; nt++)
 #pragma unroll
-      for (int i = 0; i < 4; i++) probe = fmaf(acc[nt][i], 0.f, probe);
-    if (__syncthreads_or(probe != 0.f)) {   // (NaN too)
+      for (int i = 0; i < 4; i++) most = most_of(most, acc[nt][i]);
+    // dW1 from their features and dL/da1
+    if (!__syncthreads_or(!(most < kSplitMost))) {
+#pragma unroll
+      for (int nt = 0; nt < 8; nt++)
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+          uint32_t w[3];
+          split3(acc[nt][2 * half], acc[nt][2 * half + 1], w);
+          put_terms(nt, half, w);
+        }
+    } else {
       if (!odd) {
         for (int i = tid; i < kLmW2; i += kGradThreads) __stcg(out + i, 0.f);
         __threadfence();
@@ -1432,23 +1472,19 @@ lm_grad_kernel(const float* __restrict__ params, const lm_block_t* __restrict__ 
 #pragma unroll
       for (int nt = 0; nt < 8; nt++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          float& d = acc[nt][i];
-          if (!f_finite(d)) lm_odd_gradient(G, out, row0 + g + 8 * (i >> 1), 8 * nt + 2 * t + (i & 1), d);
-          d = f_finite(d) ? d : 0.f;
+        for (int half = 0; half < 2; half++) {
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            float& d = acc[nt][2 * half + e];
+            if (f_finite(d)) continue;
+            lm_odd_gradient(G, out, row0 + g + 8 * half, 8 * nt + 2 * t + e, d);
+            d = 0.f;
+          }
+          uint32_t w[3];
+          split3_any(acc[nt][2 * half], acc[nt][2 * half + 1], w);
+          put_terms(nt, half, w);
         }
     }
-    // dW1 from their features and dL/da1
-#pragma unroll
-    for (int nt = 0; nt < 8; nt++)
-#pragma unroll
-      for (int half = 0; half < 2; half++) {
-        uint32_t w[3];
-        split3(acc[nt][2 * half], acc[nt][2 * half + 1], w);
-#pragma unroll
-        for (int s = 0; s < 3; s++)
-          *reinterpret_cast<uint32_t*>(&G.d[s][row0 + g + 8 * half][8 * nt + 2 * t]) = w[s];
-      }
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < kMine1; u++) {

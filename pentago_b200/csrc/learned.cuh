@@ -124,13 +124,11 @@ PG_HD uint32_t f_raw(float f) {
 #endif
 }
 PG_HD float bf16_value(uint16_t h) { return f_bits(uint32_t(h) << 16); }
-// Round to nearest even; bf16_round_number of a number, which is quicker
-// (NaN's bits would wrap to 0 there).
-PG_HD uint16_t bf16_round_number(float f) {
+// Round to nearest even; NaN stays NaN (rounded as a number its bits could wrap to 0).
+PG_HD uint16_t bf16_round(float f) {
   const uint32_t u = f_raw(f);
-  return uint16_t((u + 0x7fffu + ((u >> 16) & 1u)) >> 16);
+  return uint16_t(f == f ? (u + 0x7fffu + ((u >> 16) & 1u)) >> 16 : u >> 16 | 0x40u);
 }
-PG_HD uint16_t bf16_round(float f) { return f == f ? bf16_round_number(f) : uint16_t(f_raw(f) >> 16 | 0x40u); }
 PG_HD bool f_finite(float f) { return (f_raw(f) & 0x7fffffffu) < 0x7f800000u; }
 PG_HD float relu(float a) { return a > 0.f ? a : 0.f; }
 
